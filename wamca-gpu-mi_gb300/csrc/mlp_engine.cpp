@@ -583,6 +583,7 @@ int JobSet::init() {
     }
   }
   MLP_CUDA(configure_merge(merge_smem_ ? merge_smem_bytes(max_size_) : 0), "configure merge");
+  MLP_CUDA(configure_small(), "configure search");
   MLP_CUDA(cudaMallocHost(&hstats_, sizeof(int64_t) * kStatWords * jobs_.size()), "cudaMallocHost");
   MLP_CUDA(cudaMallocHost(&hstats2_, sizeof(int64_t) * kStatWords * jobs_.size()), "cudaMallocHost");
   for (int b = 0; b < 2; b++) {
@@ -902,6 +903,19 @@ int JobSet::enqueue_iterations(int iters) {
 // pass leaves the rest of it as kernels that return at once.
 constexpr int kDeviceLoopBody = 16;
 
+// Every delta of the search fits 32 bits: costs are below dmax * size^2 / 2,
+// so a 64-bit job's deltas are the 32-bit ones, exactly.
+static bool fits32(const Job* j) { return (int64_t)j->prob->dmax * j->size * j->size <= INT32_MAX; }
+
+// The one-launch search applies: one search over all neighbourhoods, with the
+// default merge and sweep, whose distances fit a CTA's shared memory.
+bool JobSet::small_search() const {
+  if (all_jobs_.size() != 1 || total_ || mask_ != 0x1f || merge_mode_ != kMergeAuto || sweep_variant_ != 1) return false;
+  const Job* j = all_jobs_[0];
+  if (j->dev.flags & kFlagRecordMoves) return false;
+  return small_fits(j->size) && (!wide_ || fits32(j));
+}
+
 int JobSet::enqueue_device_loop(int max_iters) {
   if (max_iters <= 0) {
     set_error("max_iters must be positive");
@@ -910,6 +924,10 @@ int JobSet::enqueue_device_loop(int max_iters) {
   if (stream_ == 0) {
     set_error("the device-side loop needs a non-default stream");
     return kErrState;
+  }
+  if (small_search()) {
+    MLP_CUDA(launch_dvnd_small(djobs_, max_size_, wide_, max_iters, stream_), "search kernel");
+    return kOk;
   }
   const int unroll = kDeviceLoopBody;
   if (!loop_graph_ || loop_unroll_ != unroll) {
@@ -1074,9 +1092,10 @@ int JobSet::check_stats(const int64_t* hst) {
   for (size_t q = 0; q < all_jobs_.size(); q++) err |= hst[q * kStatWords + kStatError];
   if (err) {
     static const char* what[] = {"", "", "merge stage-2 hand-off timed out (no longer produced)", "kept-move region overflow",
-                                 "TOTAL list overflow", "TOTAL selection invariant broken"};
+                                 "TOTAL list overflow", "TOTAL selection invariant broken",
+                                 "distance rows did not arrive in shared memory"};
     set_error(std::string("device reported an internal error (code ") + std::to_string(err) + ": " +
-              (err >= 2 && err <= 5 ? what[err] : "unknown") + ")");
+              (err >= 2 && err <= 6 ? what[err] : "unknown") + ")");
     return kErrState;
   }
   return kOk;

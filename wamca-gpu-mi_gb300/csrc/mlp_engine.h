@@ -186,6 +186,7 @@ class JobSet {
   // every tile instead of having the ADS rebuild (one CTA, on the merge's
   // critical path) write term tables.
   bool local_terms() const { return all_jobs_.size() == 1; }
+  bool small_search() const;
   int graph_for(int iters, cudaGraphExec_t* out);
   std::vector<Job*> all_jobs_;  // every job of the set (statistics order)
   std::vector<Job*> jobs_;      // the jobs the launches cover

@@ -103,6 +103,12 @@ cudaError_t launch_total_finish(const JobDev* jobs, int njobs, bool wide, bool u
                                 cudaStream_t s);
 // Opt the TOTAL greedy into its dynamic shared memory (configure_merge calls it).
 cudaError_t configure_total();
+// A whole DVND (all five neighbourhoods, 32-bit deltas) of one small search in
+// one launch (mlp_small.cu): the job's tour, arrays and statistics afterwards
+// are those of the iterated sweep and merge.
+bool small_fits(int size);
+cudaError_t configure_small();
+cudaError_t launch_dvnd_small(const JobDev* job, int size, bool wide, int64_t limit, cudaStream_t s);
 // MLSolution::random on the device (mlp_grasp.cu): one start per task, its
 // n + 1 entries written to `tour` (device), MTRandom seeded with `seed`;
 // alpha in [0, 1].  ties = 0: equal distances ordered by client id (one warp
