@@ -487,18 +487,23 @@ int build_random_tours(const std::vector<GraspTask>& tasks, cudaStream_t stream)
   struct Buffers {  // stream-ordered: no device-wide synchronisation
     cudaStream_t st;
     GraspTask* tasks = nullptr;
+    GraspSortJob* sorts = nullptr;
+    uint16_t* table = nullptr;
     int* err = nullptr;
     uint32_t* scratch = nullptr;
     ~Buffers() {
-      if (tasks) cudaFreeAsync(tasks, st);
-      if (err) cudaFreeAsync(err, st);
-      if (scratch) cudaFreeAsync(scratch, st);
+      for (void* p : {(void*)tasks, (void*)sorts, (void*)table, (void*)err, (void*)scratch})
+        if (p) cudaFreeAsync(p, st);
     }
   } b{stream};
   // Canonical-tie tasks first, then the reference-tie ones (one launch each);
-  // the latter above kGraspRefSmemN nodes get 2n words of scratch.
+  // the former share one set of ordered rows per distance matrix, the latter
+  // above kGraspRefSmemN nodes get 2n words of scratch.
   std::vector<GraspTask> order;
-  int64_t words = 0;
+  std::vector<GraspSortJob> sorts;
+  std::map<const int32_t*, int64_t> rows_of;
+  int64_t words = 0, entries = 0, nrows = 0;
+  int max_n = 0;
   for (int pass = 0; pass < 2; pass++)
     for (GraspTask t : tasks) {
       if (t.n < 1 || t.n > kMaxSize - 1 || !t.D || !t.tour || t.ties < 0 || t.ties > 1) {
@@ -507,7 +512,16 @@ int build_random_tours(const std::vector<GraspTask>& tasks, cudaStream_t stream)
       }
       if (t.ties != pass) continue;
       t.scratch = 0;
-      if (t.ties && t.n > kGraspRefSmemN) {
+      if (!t.ties) {
+        const auto at = rows_of.emplace(t.D, entries);
+        if (at.second) {
+          sorts.push_back(GraspSortJob{t.D, entries, nrows, t.n, 0});
+          entries += (int64_t)t.n * t.n;
+          nrows += t.n;
+          max_n = std::max(max_n, t.n);
+        }
+        t.scratch = at.first->second;
+      } else if (t.n > kGraspRefSmemN) {
         t.scratch = words;
         words += 2 * (int64_t)t.n;
       }
@@ -524,9 +538,20 @@ int build_random_tours(const std::vector<GraspTask>& tasks, cudaStream_t stream)
                            stream),
            "copy constructor tasks");
   MLP_CUDA(cudaMemsetAsync(b.err, 0, sizeof(int), stream), "memset(constructor flag)");
-  MLP_CUDA(launch_grasp(b.tasks, ncanon, 0, nullptr, b.err, stream), "constructor kernel");
-  MLP_CUDA(launch_grasp(b.tasks + ncanon, (int)order.size() - ncanon, 1, b.scratch, b.err, stream),
-           "constructor kernel");
+  if (ncanon > 0) {
+    // Without room for the ordered rows the starts select from unsorted ones.
+    if (cudaMallocAsync(&b.table, sizeof(uint16_t) * (size_t)entries, stream) != cudaSuccess) {
+      cudaGetLastError();
+      b.table = nullptr;
+    } else {
+      MLP_CUDA(cudaMallocAsync(&b.sorts, sizeof(GraspSortJob) * sorts.size(), stream), "cudaMallocAsync(constructor rows)");
+      MLP_CUDA(cudaMemcpyAsync(b.sorts, sorts.data(), sizeof(GraspSortJob) * sorts.size(), cudaMemcpyHostToDevice, stream),
+               "copy constructor rows");
+      MLP_CUDA(launch_grasp_sort(b.sorts, (int)sorts.size(), nrows, max_n, b.table, stream), "constructor rows kernel");
+    }
+    MLP_CUDA(launch_grasp(b.tasks, ncanon, max_n, b.table, b.err, stream), "constructor kernel");
+  }
+  MLP_CUDA(launch_grasp_ref(b.tasks + ncanon, (int)order.size() - ncanon, b.scratch, stream), "constructor kernel");
   int herr = 0;
   MLP_CUDA(cudaMemcpyAsync(&herr, b.err, sizeof(int), cudaMemcpyDeviceToHost, stream), "read constructor flag");
   MLP_CUDA(cudaStreamSynchronize(stream), "constructor");

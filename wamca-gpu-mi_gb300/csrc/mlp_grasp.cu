@@ -10,13 +10,23 @@
 // rank is taken in (distance, client id) order.  costTour: depot 0 closes the
 // tour.
 //
-// One warp builds one start.  MT19937 (source/mtrand.cpp:52-124) runs on
-// lane 0 with its state in shared memory.  Each step selects rank r among the
-// remaining candidates with a three-level radix select (10-bit digits of the
-// 30-bit key distance << 14 | id) over a per-warp 1024-bin histogram.  Up to
-// 2048 nodes the candidates and the step's keys stay in shared memory (one
-// distance gather per candidate and step); larger instances keep the
-// candidates in the tail of the tour being built and gather in every pass.
+// One warp builds one start.  MT19937 (source/mtrand.cpp:52-124) has its state
+// in shared memory.  The draws depend on the step's number alone, so a warp
+// makes those of 32 steps at once.
+//
+// k_grasp_sort orders every client's row by (distance, id) once per call, and
+// a step of k_grasp takes the r-th client of its row that is not in the tour
+// yet: it walks the row 256 clients at a time, a ballot over the visited
+// bitmap per 32, and stops where the count passes r.  A step is then one L2
+// round trip and about 150 instructions a warp (1.0 us at n = 1000); selecting
+// the rank among unsorted keys (k_grasp_select, three histogram passes a step)
+// takes 8.7 us a step and holds 23 KB of shared memory a warp.  A whole call at
+// n = 1000, unsorted -> ordered rows: one start 8.9 -> 1.25 ms, 512 starts
+// 9.5 -> 1.23, 2048 starts 18.7 -> 1.66; 4 starts at n = 5000 535 -> 15.6.
+// The sort is bound by its shared-memory passes (23 us at n = 1000), a start by
+// the chain of its steps.
+// The ordered rows take 2 n^2 bytes of scratch; where that cannot be allocated
+// k_grasp_select serves.
 #include <cmath>
 #include <cstdint>
 
@@ -29,7 +39,8 @@ namespace mlp {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kGraspWarps = 8;     // starts per CTA
+constexpr int kGraspWarps = 8;     // starts per CTA of k_grasp_select
+constexpr int kGraspSortedWarps = 4;  // and of k_grasp
 constexpr int kGraspSmemN = 2048;  // up to this n a step's keys stay in shared memory
 constexpr int kMtN = 624, kMtM = 397;
 
@@ -42,46 +53,183 @@ struct GraspSmem {
   static constexpr size_t total = per_warp * kGraspWarps;
 };
 
-// MTRandom::seed (mtrand.cpp:52-61)
+// MTRandom::seed (mtrand.cpp:52-61), by one lane.
 __device__ void mt_seed(uint32_t* st, uint32_t s) {
   st[0] = s;
-  for (int p = 1; p < kMtN; p++) st[p] = 1812433253u * (st[p - 1] ^ (st[p - 1] >> 30)) + (uint32_t)p;
+  for (int p = 1; p < kMtN; p++) {
+    s = 1812433253u * (s ^ (s >> 30)) + (uint32_t)p;
+    st[p] = s;
+  }
 }
 
-// MTRandom::gen (mtrand.cpp:99-124)
+// MTRandom::gen (mtrand.cpp:99-124), by a warp: word i depends on words i,
+// i + 1 and i + 397 (mod 624) of its own time, so 32 words in a row can be
+// renewed together, all read before any is written.
 __device__ void mt_gen(uint32_t* st) {
-  int i = 0;
-  uint32_t y;
-  for (; i < kMtN - kMtM; i++) {
-    y = (st[i] & 0x80000000u) | (st[i + 1] & 0x7fffffffu);
-    st[i] = st[i + kMtM] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+  const int lane = threadIdx.x & 31;
+  for (int i0 = 0; i0 < kMtN; i0 += 32) {
+    const int i = i0 + lane;
+    uint32_t v = 0;
+    if (i < kMtN) {
+      const uint32_t y = (st[i] & 0x80000000u) | (st[i + 1 < kMtN ? i + 1 : 0] & 0x7fffffffu);
+      v = st[i + kMtM < kMtN ? i + kMtM : i + kMtM - kMtN] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
+    }
+    __syncwarp();
+    if (i < kMtN) st[i] = v;
+    __syncwarp();
   }
-  for (; i < kMtN - 1; i++) {
-    y = (st[i] & 0x80000000u) | (st[i + 1] & 0x7fffffffu);
-    st[i] = st[i + (kMtM - kMtN)] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
-  }
-  y = (st[kMtN - 1] & 0x80000000u) | (st[0] & 0x7fffffffu);
-  st[kMtN - 1] = st[kMtM - 1] ^ (y >> 1) ^ ((y & 1u) ? 0x9908b0dfu : 0u);
 }
 
-// MTRandom::rand() with tempering (mtrand.h:167-179); *pos is the state index.
-__device__ uint32_t mt_rand(uint32_t* st, int* pos) {
-  if (*pos >= kMtN) {
-    mt_gen(st);
-    *pos = 0;
-  }
-  uint32_t x = st[(*pos)++];
+// MTRandom::rand() with tempering (mtrand.h:167-179) of state word x.
+__device__ __forceinline__ uint32_t mt_temper(uint32_t x) {
   x ^= (x >> 11);
   x ^= (x << 7) & 0x9d2c5680u;
   x ^= (x << 15) & 0xefc60000u;
   return x ^ (x >> 18);
 }
 
-// MTRandom::rand(max) (mtrand.h:193-195): IEEE double multiply and divide,
-// as on the host.
-__device__ uint32_t mt_rand_max(uint32_t* st, int* pos, uint32_t mx) {
-  const double v = __dmul_rn((double)mx + 1.0, (double)mt_rand(st, pos));
-  return (uint32_t)__ddiv_rn(v, 4294967296.0);
+// MTRandom::rand(max) (mtrand.h:193-195) from the draw x: IEEE double multiply
+// and divide, as on the host (the divisor is 2^32, so the product with 2^-32
+// is the quotient exactly).
+__device__ __forceinline__ uint32_t mt_scale(uint32_t x, uint32_t mx) {
+  const double v = __dmul_rn((double)mx + 1.0, (double)x);
+  return (uint32_t)__dmul_rn(v, 1.0 / 4294967296.0);
+}
+
+// The draws of a start's steps, 32 at a time: lane l of draw(k0) returns the
+// rank of the step with n - 1 - (k0 + l) clients left after it.  Every lane of
+// the warp calls it, with k0 = 0, 32, 64, ...
+struct GraspDraws {
+  uint32_t* st;
+  int n, pos;
+  float alpha;
+  __device__ __forceinline__ uint32_t draw(int k0) {
+    const int lane = threadIdx.x & 31, cnt = n - 1 - k0 - lane;
+    // A draw is made while more than one candidate remains and the restricted
+    // list is not empty (alpha > 0).
+    const uint32_t rcl = cnt > 1 ? (uint32_t)ceilf(__fmul_rn(alpha, (float)cnt)) : 0u;
+    uint32_t x = 0;
+    const int left = kMtN - pos;
+    if (lane < left) x = st[pos + lane];
+    if (left < 32) {
+      __syncwarp();
+      mt_gen(st);
+      if (lane >= left) x = st[lane - left];
+      pos = 32 - left;
+    } else {
+      pos += 32;
+    }
+    const uint32_t r = rcl > 0 ? mt_scale(mt_temper(x), rcl - 1) : 0u;
+    return cnt > 0 && r >= (uint32_t)cnt ? (uint32_t)(cnt - 1) : r;  // alpha <= 1 (checked by the host) keeps r < cnt
+  }
+};
+
+// Ordered rows: row c of a job holds the n client ids in (distance to c, id)
+// order, as 16-bit words.  One CTA per row, a bitonic sort in shared memory.
+__global__ void __launch_bounds__(1024) k_grasp_sort(const GraspSortJob* __restrict__ jobs, int njobs,
+                                                     uint16_t* __restrict__ out) {
+  extern __shared__ __align__(16) uint8_t gsm[];
+  uint32_t* key = (uint32_t*)gsm;
+  int lo = 0, hi = njobs - 1;  // the job whose rows hold this CTA's
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (jobs[mid].row0 <= (int64_t)blockIdx.x) lo = mid;
+    else hi = mid - 1;
+  }
+  const GraspSortJob job = jobs[lo];
+  const int n = job.n, c = (int)((int64_t)blockIdx.x - job.row0), tid = threadIdx.x, nt = blockDim.x;
+  int P = 1;
+  while (P < n) P <<= 1;
+  const int32_t* __restrict__ row = job.D + (size_t)c * n;
+  for (int q = tid; q < P; q += nt) key[q] = q < n ? ((uint32_t)row[q] << 14) | (uint32_t)q : 0xffffffffu;
+  for (int k = 2; k <= P; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      __syncthreads();
+      for (int q = tid; q < (P >> 1); q += nt) {
+        const int a = 2 * q - (q & (j - 1)), b = a + j;
+        const uint32_t x = key[a], y = key[b];
+        if ((x > y) == ((a & k) == 0)) {
+          key[a] = y;
+          key[b] = x;
+        }
+      }
+    }
+  __syncthreads();
+  uint16_t* o = out + job.out + (size_t)c * n;
+  for (int q = tid; q < n; q += nt) o[q] = (uint16_t)(key[q] & 0x3fffu);
+}
+
+// One start per warp over the ordered rows.
+constexpr int kGraspGroup = 8;  // ballots of 32 clients looked at together
+__global__ void __launch_bounds__(32 * kGraspSortedWarps)
+    k_grasp(const GraspTask* __restrict__ tasks, int count, const uint16_t* __restrict__ table, int words,
+            int* __restrict__ err) {
+  extern __shared__ __align__(16) uint8_t gsm[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int start = blockIdx.x * kGraspSortedWarps + wid;
+  if (start >= count) return;  // whole warps only
+  const GraspTask task = tasks[start];
+  const int n = task.n;
+  const uint16_t* __restrict__ rows = table + task.scratch;
+  uint32_t* st = (uint32_t*)gsm + (size_t)wid * (kMtN + words);
+  uint32_t* seen = st + kMtN;  // clients in the tour (and past the last one)
+  int32_t* t = task.tour;
+  if (lane == 0) {
+    mt_seed(st, task.seed);
+    t[0] = 0;
+    t[n] = 0;
+  }
+  for (int w = lane; w < words; w += 32) seen[w] = w == 0 ? 1u : 0u;
+  __syncwarp();
+  GraspDraws draws{st, n, kMtN, task.alpha};
+  int last = 0;
+  for (int k0 = 0; k0 < n - 1; k0 += 32) {
+    const uint32_t rk = draws.draw(k0);
+    const int steps = min(32, n - 1 - k0);
+    int32_t mine = 0;
+    for (int k = 0; k < steps; k++) {
+      uint32_t r = __shfl_sync(kFull, rk, k);
+      const uint16_t* __restrict__ row = rows + (size_t)last * n;
+      int cur = -1;
+      uint32_t id[kGraspGroup], nx[kGraspGroup];
+#pragma unroll
+      for (int u = 0; u < kGraspGroup; u++) id[u] = 32 * u + lane < n ? row[32 * u + lane] : 0u;  // client 0 is in the tour
+      for (int p0 = 0; p0 < n; p0 += 32 * kGraspGroup) {
+#pragma unroll
+        for (int u = 0; u < kGraspGroup; u++) {
+          const int p = p0 + 32 * (kGraspGroup + u) + lane;
+          nx[u] = p < n ? row[p] : 0u;
+        }
+        unsigned bal[kGraspGroup];
+#pragma unroll
+        for (int u = 0; u < kGraspGroup; u++) bal[u] = __ballot_sync(kFull, !((seen[id[u] >> 5] >> (id[u] & 31u)) & 1u));
+#pragma unroll
+        for (int u = 0; u < kGraspGroup; u++) {
+          const uint32_t c = (uint32_t)__popc(bal[u]);
+          if (cur < 0) {
+            if (r < c) {
+              const bool hit = ((bal[u] >> lane) & 1u) && (uint32_t)__popc(bal[u] & ((1u << lane) - 1u)) == r;
+              cur = (int)__shfl_sync(kFull, id[u], __ffs(__ballot_sync(kFull, hit)) - 1);
+            } else {
+              r -= c;
+            }
+          }
+        }
+        if (cur >= 0) break;
+#pragma unroll
+        for (int u = 0; u < kGraspGroup; u++) id[u] = nx[u];
+      }
+      if (cur < 0) {  // unreachable: r < the number of clients left
+        if (lane == 0) atomicAdd(err, 1);
+        return;
+      }
+      if (lane == 0) seen[cur >> 5] |= 1u << (cur & 31);
+      if (lane == k) mine = cur;
+      last = cur;
+      __syncwarp();
+    }
+    if (lane < steps) t[1 + k0 + lane] = mine;
+  }
 }
 
 __device__ __forceinline__ uint32_t grasp_key(const int32_t* __restrict__ row, int32_t c) {
@@ -151,8 +299,12 @@ __device__ int find_key(int cnt, uint32_t key, KeyOf key_of) {
   return -1;
 }
 
+// One start per warp from the unsorted rows (no scratch): each step selects
+// rank r among the remaining candidates with a three-level radix select
+// (10-bit digits of the 30-bit key distance << 14 | id) over a per-warp
+// 1024-bin histogram.
 __global__ void __launch_bounds__(32 * kGraspWarps)
-    k_grasp(const GraspTask* __restrict__ tasks, int count, int* __restrict__ err) {
+    k_grasp_select(const GraspTask* __restrict__ tasks, int count, int* __restrict__ err) {
   extern __shared__ __align__(16) uint8_t gsm[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int start = blockIdx.x * kGraspWarps + wid;
@@ -160,7 +312,6 @@ __global__ void __launch_bounds__(32 * kGraspWarps)
   const GraspTask task = tasks[start];
   const int32_t* __restrict__ D = task.D;
   const int n = task.n;
-  const float alpha = task.alpha;
   uint8_t* base = gsm + wid * GraspSmem::per_warp;
   uint32_t* st = (uint32_t*)(base + GraspSmem::mt);
   uint32_t* hist = (uint32_t*)(base + GraspSmem::hist);
@@ -171,7 +322,6 @@ __global__ void __launch_bounds__(32 * kGraspWarps)
   // shared memory and their keys are gathered once per step; above, they
   // are t[len..n) and every pass gathers the keys again.
   const bool smem = n <= kGraspSmemN;
-  int pos = kMtN;
   if (lane == 0) mt_seed(st, task.seed);
   if (smem) {
     for (int q = lane; q < n - 1; q += 32) ids[q] = q + 1;
@@ -183,16 +333,13 @@ __global__ void __launch_bounds__(32 * kGraspWarps)
     t[n] = 0;
   }
   __syncwarp();
+  GraspDraws draws{st, n, kMtN, task.alpha};
+  uint32_t rk = 0;
   int last = 0;
   for (int len = 1; len < n; len++) {
     const int cnt = n - len;
-    uint32_t r = 0;
-    if (lane == 0 && cnt > 1) {
-      const uint32_t rcl = (uint32_t)ceilf(__fmul_rn(alpha, (float)cnt));
-      r = rcl > 0 ? mt_rand_max(st, &pos, rcl - 1) : 0u;
-    }
-    r = __shfl_sync(kFull, r, 0);
-    if (r >= (uint32_t)cnt) r = cnt - 1;  // alpha <= 1 (checked by the host) keeps r < cnt
+    if (((len - 1) & 31) == 0) rk = draws.draw(len - 1);
+    const uint32_t r = __shfl_sync(kFull, rk, (len - 1) & 31);
     const int32_t* __restrict__ row = D + (size_t)last * n;
     uint32_t key;
     int q;
@@ -245,8 +392,7 @@ __global__ void __launch_bounds__(32)
   const GraspTask task = tasks[blockIdx.x];
   const int32_t* __restrict__ D = task.D;
   const int n = task.n;
-  const float alpha = task.alpha;
-  const bool desc = alpha < 0.5f;
+  const bool desc = task.alpha < 0.5f;
   int32_t* t = task.tour;
   uint32_t* st = (uint32_t*)gsm;
   uint32_t* keys;
@@ -258,7 +404,6 @@ __global__ void __launch_bounds__(32)
     keys = scratch + task.scratch;
     ids = (int32_t*)(keys + n);
   }
-  int pos = kMtN;
   if (lane == 0) {
     mt_seed(st, task.seed);
     t[0] = 0;
@@ -266,15 +411,14 @@ __global__ void __launch_bounds__(32)
   }
   for (int q = lane; q < n - 1; q += 32) ids[q] = q + 1;
   __syncwarp();
+  GraspDraws draws{st, n, kMtN, task.alpha};
+  uint32_t rk = 0;
   int last = 0;
   for (int len = 1; len < n; len++) {
     const int cnt = n - len;
-    uint32_t idx = 0;
+    if (((len - 1) & 31) == 0) rk = draws.draw(len - 1);
+    uint32_t idx = __shfl_sync(kFull, rk, (len - 1) & 31);
     if (cnt > 1) {
-      if (lane == 0) {
-        const uint32_t rcl = (uint32_t)ceilf(__fmul_rn(alpha, (float)cnt));
-        idx = rcl > 0 ? mt_rand_max(st, &pos, rcl - 1) : 0u;
-      }
       const int32_t* __restrict__ row = D + (size_t)last * n;
       for (int x = lane; x < cnt; x += 32) keys[x] = (uint32_t)row[ids[x]];
       __syncwarp();
@@ -298,21 +442,42 @@ __global__ void __launch_bounds__(32)
 }  // namespace
 
 cudaError_t configure_grasp() {
-  cudaError_t e = cudaFuncSetAttribute(k_grasp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GraspSmem::total);
+  cudaError_t e = cudaFuncSetAttribute(k_grasp_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GraspSmem::total);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_grasp_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kMaxSize);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(k_grasp_ref, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGraspRefSmem);
 }
 
-cudaError_t launch_grasp(const GraspTask* tasks, int count, int ties, uint32_t* scratch, int* err, cudaStream_t s) {
+cudaError_t launch_grasp_sort(const GraspSortJob* jobs, int njobs, int64_t nrows, int max_n, uint16_t* table, cudaStream_t s) {
+  if (nrows <= 0) return cudaSuccess;
+  const cudaError_t e = configure_grasp();
+  if (e != cudaSuccess) return e;
+  int P = 1;
+  while (P < max_n) P <<= 1;
+  k_grasp_sort<<<(unsigned)nrows, P <= 2048 ? 256 : 1024, 4 * (size_t)P, s>>>(jobs, njobs, table);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_grasp(const GraspTask* tasks, int count, int max_n, const uint16_t* table, int* err, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
   const cudaError_t e = configure_grasp();
   if (e != cudaSuccess) return e;
-  if (ties) {
-    k_grasp_ref<<<count, 32, kGraspRefSmem, s>>>(tasks, scratch);
-    return cudaGetLastError();
+  if (table == nullptr) {
+    k_grasp_select<<<(count + kGraspWarps - 1) / kGraspWarps, 32 * kGraspWarps, GraspSmem::total, s>>>(tasks, count, err);
+  } else {
+    const int words = (max_n + 31) / 32;
+    k_grasp<<<(count + kGraspSortedWarps - 1) / kGraspSortedWarps, 32 * kGraspSortedWarps,
+              4 * (size_t)(kMtN + words) * kGraspSortedWarps, s>>>(tasks, count, table, words, err);
   }
-  const int grid = (count + kGraspWarps - 1) / kGraspWarps;
-  k_grasp<<<grid, 32 * kGraspWarps, GraspSmem::total, s>>>(tasks, count, err);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_grasp_ref(const GraspTask* tasks, int count, uint32_t* scratch, cudaStream_t s) {
+  if (count <= 0) return cudaSuccess;
+  const cudaError_t e = configure_grasp();
+  if (e != cudaSuccess) return e;
+  k_grasp_ref<<<count, 32, kGraspRefSmem, s>>>(tasks, scratch);
   return cudaGetLastError();
 }
 
