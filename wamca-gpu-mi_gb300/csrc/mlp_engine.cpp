@@ -570,12 +570,15 @@ JobSet::~JobSet() {
   for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second);
   if (loop_graph_) cudaGraphExecDestroy(loop_graph_);
   if (djobs_) cudaFree(djobs_);
-  if (dtiles_) cudaFree(dtiles_);
+  for (TileList& l : lists_) {
+    if (l.d) cudaFree(l.d);
+    for (SweepTile* h : l.h)
+      if (h) cudaFreeHost(h);
+  }
   if (hstats_) cudaFreeHost(hstats_);
   if (hstats2_) cudaFreeHost(hstats2_);
   for (int b = 0; b < 2; b++) {
     if (stats_ev_[b]) cudaEventDestroy(stats_ev_[b]);
-    if (htiles_[b]) cudaFreeHost(htiles_[b]);
     if (hjobs_[b]) cudaFreeHost(hjobs_[b]);
   }
   if (dstats_) cudaFree(dstats_);
@@ -629,36 +632,35 @@ int JobSet::init() {
            "copy jobs");
   MLP_CUDA(cudaStreamSynchronize(stream_), "copy jobs");
   if (shape_ < 0) shape_ = default_shape(max_size_, (int)jobs_.size());
-  return build_tiles();
+  return small_search() ? kOk : ensure_tiles(dvnd_list());  // a one-launch search has no list
 }
 
-int JobSet::build_tiles(int buf, bool sync) {
-  const TileShape ts = kTileShapes[shape_];
+int JobSet::ensure_tiles(int list, int buf, bool sync) {
+  TileList& l = lists_[list];
+  if (l.ok) return kOk;
+  const TileShape ts = kTileShapes[list == 1 ? wide_shape(shape_) : shape_];
   size_t count = 0;
   for (size_t q = 0; q < jobs_.size(); q++) {
     const int sz = jobs_[q]->size;
     for (int rb = 0; rb < sweep_row_blocks(sz, ts.tr); rb++) count += (size_t)sweep_row_tiles(sz, 1 + rb * ts.tr, ts.tl);
   }
-  for (auto& kv : graphs_) cudaGraphExecDestroy(kv.second);
-  graphs_.clear();
-  if (loop_graph_) cudaGraphExecDestroy(loop_graph_);
-  loop_graph_ = nullptr;
-  if (count > tiles_cap_ || dtiles_ == nullptr) {
-    // Grow (the set's first build, or more jobs or smaller tiles than before).
+  drop_graphs();
+  if (count > l.cap || l.d == nullptr) {
+    // Grow (the list's first build, or more jobs or smaller tiles than before).
     MLP_CUDA(cudaStreamSynchronize(stream_), "grow tiles");
-    if (dtiles_) cudaFree(dtiles_);
-    dtiles_ = nullptr;
+    if (l.d) cudaFree(l.d);
+    l.d = nullptr;
     for (int b = 0; b < 2; b++) {
-      if (htiles_[b]) cudaFreeHost(htiles_[b]);
-      htiles_[b] = nullptr;
+      if (l.h[b]) cudaFreeHost(l.h[b]);
+      l.h[b] = nullptr;
     }
-    tiles_cap_ = 0;
+    l.cap = 0;
     const size_t cap = std::max<size_t>(1, count);
-    MLP_CUDA(cudaMalloc(&dtiles_, sizeof(SweepTile) * cap), "cudaMalloc(tiles)");
-    for (int b = 0; b < 2; b++) MLP_CUDA(cudaMallocHost(&htiles_[b], sizeof(SweepTile) * cap), "cudaMallocHost(tiles)");
-    tiles_cap_ = cap;
+    MLP_CUDA(cudaMalloc(&l.d, sizeof(SweepTile) * cap), "cudaMalloc(tiles)");
+    for (int b = 0; b < 2; b++) MLP_CUDA(cudaMallocHost(&l.h[b], sizeof(SweepTile) * cap), "cudaMallocHost(tiles)");
+    l.cap = cap;
   }
-  SweepTile* h = htiles_[buf];
+  SweepTile* h = l.h[buf];
   size_t k = 0;
   for (size_t q = 0; q < jobs_.size(); q++) {
     const int sz = jobs_[q]->size;
@@ -667,10 +669,11 @@ int JobSet::build_tiles(int buf, bool sync) {
       for (int c = 0; c < sweep_row_tiles(sz, r0, ts.tl); c++) h[k++] = SweepTile{(int32_t)q, r0, 1 + c * ts.tl, 0};
     }
   }
-  ntiles_ = (int)count;
+  l.n = (int)count;
   if (count > 0)
-    MLP_CUDA(cudaMemcpyAsync(dtiles_, h, sizeof(SweepTile) * count, cudaMemcpyHostToDevice, stream_), "copy tiles");
+    MLP_CUDA(cudaMemcpyAsync(l.d, h, sizeof(SweepTile) * count, cudaMemcpyHostToDevice, stream_), "copy tiles");
   if (sync) MLP_CUDA(cudaStreamSynchronize(stream_), "copy tiles");
+  l.ok = true;
   return kOk;
 }
 
@@ -690,7 +693,8 @@ int JobSet::set_active(const std::vector<int>& idx, int buf, bool sync) {
   for (size_t q = 0; q < jobs_.size(); q++) h[q] = jobs_[q]->dev;
   MLP_CUDA(cudaMemcpyAsync(djobs_, h, sizeof(JobDev) * jobs_.size(), cudaMemcpyHostToDevice, stream_),
            "copy jobs");
-  return build_tiles(buf, sync);
+  drop_tiles();
+  return ensure_tiles(dvnd_list(), buf, sync);
 }
 
 int JobSet::ensure_all_active() {
@@ -719,7 +723,9 @@ int JobSet::set_shape(int shape) {
     return kOk;
   }
   shape_ = shape;
-  return djobs_ ? build_tiles() : kOk;
+  drop_tiles();
+  drop_graphs();
+  return djobs_ ? ensure_tiles(dvnd_list()) : kOk;
 }
 
 int JobSet::set_unroll(int u) {
@@ -807,21 +813,23 @@ int JobSet::set_total(bool on) {
     shape_ = shape_user_;
   }
   total_ = on;
-  return build_tiles();  // also drops the captured graphs
+  drop_tiles();
+  drop_graphs();
+  return ensure_tiles(dvnd_list());
 }
 
 int JobSet::launch_iteration() {
   if (total_) {
     const int nj = (int)jobs_.size();
-    MLP_CUDA(launch_sweep_collect(dtiles_, ntiles_, djobs_, wide_, shape_, stream_), "sweep kernel");
+    MLP_CUDA(launch_sweep_collect(lists_[0].d, lists_[0].n, djobs_, wide_, shape_, stream_), "sweep kernel");
     MLP_CUDA(launch_total_select(djobs_, nj, wide_, stream_), "TOTAL greedy kernel");
     MLP_CUDA(launch_total_finish(djobs_, nj, wide_, solo_smem_, max_size_, stream_), "merge kernel");
     return kOk;
   }
-  if (dvnd_sweep())
-    MLP_CUDA(launch_sweep_dvnd(dtiles_, ntiles_, djobs_, shape_, local_terms(), stream_), "sweep kernel");
-  else
-    MLP_CUDA(launch_sweep(dtiles_, ntiles_, djobs_, wide_, shape_, true, stream_), "sweep kernel");
+  {
+    const int st = launch_dvnd_sweep();
+    if (st != kOk) return st;
+  }
   if (solo_merge())
     MLP_CUDA(launch_merge_solo(djobs_, (int)jobs_.size(), wide_, solo_smem_, max_size_, stream_), "merge kernel");
   else
@@ -866,16 +874,28 @@ int JobSet::sweep_only() {
     int st = ensure_all_active();
     if (st != kOk) return st;
   }
+  {
+    const int st = ensure_tiles(0);
+    if (st != kOk) return st;
+  }
   MLP_CUDA(launch_stats_begin(djobs_, (int)jobs_.size(), 1, stream_), "stats kernel");
-  MLP_CUDA(launch_sweep(dtiles_, ntiles_, djobs_, wide_, shape_, false, stream_), "sweep kernel");
+  MLP_CUDA(launch_sweep(lists_[0].d, lists_[0].n, djobs_, wide_, shape_, false, stream_), "sweep kernel");
   return kOk;
 }
 
 int JobSet::sweep_kernel() {
-  if (dvnd_sweep())
-    MLP_CUDA(launch_sweep_dvnd(dtiles_, ntiles_, djobs_, shape_, local_terms(), stream_), "sweep kernel");
+  const int st = ensure_tiles(sweep64() ? 1 : 0);
+  return st != kOk ? st : launch_dvnd_sweep();
+}
+
+int JobSet::launch_dvnd_sweep() {
+  const TileList& l = lists_[sweep64() ? 1 : 0];
+  if (sweep64())
+    MLP_CUDA(launch_sweep_dvnd_wide(l.d, l.n, djobs_, wide_shape(shape_), stream_), "sweep kernel");
+  else if (dvnd_sweep())
+    MLP_CUDA(launch_sweep_dvnd(l.d, l.n, djobs_, shape_, local_terms(), stream_), "sweep kernel");
   else
-    MLP_CUDA(launch_sweep(dtiles_, ntiles_, djobs_, wide_, shape_, true, stream_), "sweep kernel");
+    MLP_CUDA(launch_sweep(l.d, l.n, djobs_, wide_, shape_, true, stream_), "sweep kernel");
   return kOk;
 }
 
@@ -905,6 +925,10 @@ int JobSet::graph_for(int iters, cudaGraphExec_t* out) {
 }
 
 int JobSet::enqueue_iterations(int iters) {
+  {
+    const int st = ensure_tiles(dvnd_list());
+    if (st != kOk) return st;
+  }
   if (stream_ == 0) {
     for (int q = 0; q < iters; q++) {
       int st = launch_iteration();
@@ -932,6 +956,12 @@ constexpr int kDeviceLoopBody = 16;
 // so a 64-bit job's deltas are the 32-bit ones, exactly.
 static bool fits32(const Job* j) { return (int64_t)j->prob->dmax * j->size * j->size <= INT32_MAX; }
 
+// One 64-bit search whose costs fit 32 bits takes the 32-bit sweep, whose
+// deltas modulo 2^32 are then the exact ones (n = 1000: 27.3 -> 22.5 us an
+// iteration).  A 64-bit batch has no 32-bit term tables: its sweep is the
+// 64-bit one.
+bool JobSet::sweep32() const { return !wide_ || (local_terms() && fits32(all_jobs_[0])); }
+
 // The one-launch search applies: one search over all neighbourhoods, with the
 // default merge and sweep, whose distances fit a CTA's shared memory.
 bool JobSet::small_search() const {
@@ -955,6 +985,10 @@ int JobSet::enqueue_device_loop(int max_iters) {
     return kOk;
   }
   const int unroll = kDeviceLoopBody;
+  {
+    const int st = ensure_tiles(dvnd_list());
+    if (st != kOk) return st;
+  }
   if (!loop_graph_ || loop_unroll_ != unroll) {
     if (loop_graph_) cudaGraphExecDestroy(loop_graph_);
     loop_graph_ = nullptr;
@@ -1022,6 +1056,10 @@ int JobSet::run(int max_iters, bool sync) {
     if (st != kOk || !sync) return st;
     std::vector<std::array<int64_t, kStatWords>> s;
     return read_stats(&s);
+  }
+  {
+    const int st = ensure_tiles(dvnd_list());
+    if (st != kOk) return st;
   }
   MLP_CUDA(launch_stats_begin(djobs_, (int)jobs_.size(), max_iters, stream_), "stats kernel");
   // Host-checked loop.  A single job replays CUDA graphs of `unroll`

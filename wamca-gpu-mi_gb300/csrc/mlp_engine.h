@@ -160,7 +160,6 @@ class JobSet {
   int set_active(const std::vector<int>& idx, int buf = 0, bool sync = true);
   int ensure_all_active();
   JobDev* device_jobs() const { return djobs_; }
-  int ntiles() const { return ntiles_; }
   // One DVND iteration over the current jobs (no statistics reset).
   int launch_iteration();
   // Merge kernel: kMergeAuto (one CTA per job for sets of kSoloMinJobs jobs
@@ -178,15 +177,33 @@ class JobSet {
   int sweep_kernel_variant() const { return sweep_variant_; }
 
  private:
-  int build_tiles(int buf = 0, bool sync = true);
+  // The tile list of a sweep: list 0 in the set's shape, list 1 in the shape
+  // of the 64-bit DVND sweep.  Built when first needed; set_active and
+  // set_shape invalidate them.
+  struct TileList {
+    SweepTile* d = nullptr;
+    SweepTile* h[2] = {nullptr, nullptr};  // pinned staging
+    size_t cap = 0;                        // tiles d and each staging buffer hold
+    int n = 0;
+    bool ok = false;
+  };
+  int ensure_tiles(int list, int buf = 0, bool sync = true);
+  int dvnd_list() const { return sweep64() && !total_ ? 1 : 0; }  // the list of an iteration's sweep
+  void drop_tiles() { lists_[0].ok = lists_[1].ok = false; }
   int check_stats(const int64_t* hst);  // the statistics' internal error words
   void drop_graphs();
-  bool dvnd_sweep() const { return sweep_variant_ == 1 && !wide_ && mask_ == 0x1f; }
+  // DVND iterations evaluate all five neighbourhoods from row and column terms:
+  // in 32 bits (32-bit jobs, and one 64-bit search whose costs fit 32 bits) or
+  // in 64.
+  bool dvnd_sweep() const { return sweep_variant_ == 1 && mask_ == 0x1f; }
+  bool sweep32() const;
+  bool sweep64() const { return dvnd_sweep() && !sweep32(); }
   // A set of one search computes the DVND sweep's row and column terms in
   // every tile instead of having the ADS rebuild (one CTA, on the merge's
   // critical path) write term tables.
   bool local_terms() const { return all_jobs_.size() == 1; }
   bool small_search() const;
+  int launch_dvnd_sweep();
   int graph_for(int iters, cudaGraphExec_t* out);
   std::vector<Job*> all_jobs_;  // every job of the set (statistics order)
   std::vector<Job*> jobs_;      // the jobs the launches cover
@@ -204,13 +221,10 @@ class JobSet {
   int sweep_variant_ = 1;
   int shape_user_ = -1;  // tile shape to restore when TOTAL mode ends
   JobDev* djobs_ = nullptr;
-  SweepTile* dtiles_ = nullptr;
-  int ntiles_ = 0;
+  TileList lists_[2];
   int64_t* hstats_ = nullptr;  // pinned, kStatWords per job
   int64_t* hstats2_ = nullptr;  // a second one (the batch loop reads one while the other fills)
   cudaEvent_t stats_ev_[2] = {nullptr, nullptr};
-  size_t tiles_cap_ = 0;                        // tiles dtiles_ and each staging buffer hold
-  SweepTile* htiles_[2] = {nullptr, nullptr};  // pinned staging of the tile list
   JobDev* hjobs_[2] = {nullptr, nullptr};      // pinned staging of the job descriptors
   int64_t* dstats_ = nullptr;  // device, kStatWords per job (jobs' stats live here)
   std::vector<void*> extra_ws_;  // merge workspaces allocated for jobs of mixed-size sets

@@ -96,6 +96,14 @@ inline int total_shape(int max_size) { return max_size <= 2000 ? kTotalShapeSmal
 // the prefix arrays (jobs whose descriptors carry no tables).
 cudaError_t launch_sweep_dvnd(const SweepTile* tiles, int ntiles, const JobDev* jobs, int shape, bool local,
                               cudaStream_t s);
+// The same for 64-bit jobs (mlp_sweep_wide.cu), terms computed per tile, two
+// diagonals a thread.  Its tile shapes: 16 rows of 128 diagonals for the shapes
+// of 16 rows or more (n = 10,000: 128 x 16 517 us, 128 x 8 599, 64 x 8 683,
+// 64 x 16 788, 64 x 4 880), else the shape's rows of at least 64 diagonals.
+constexpr int wide_shape(int shape) {
+  return kTileShapes[shape].tr >= 16 ? 7 : kTileShapes[shape].tl == 128 ? 6 : kTileShapes[shape].tr == 8 ? 4 : 3;
+}
+cudaError_t launch_sweep_dvnd_wide(const SweepTile* tiles, int ntiles, const JobDev* jobs, int shape, cudaStream_t s);
 cudaError_t launch_sweep_collect(const SweepTile* tiles, int ntiles, const JobDev* jobs, bool wide, int shape,
                                  cudaStream_t s);
 cudaError_t launch_total_select(const JobDev* jobs, int njobs, bool wide, cudaStream_t s);

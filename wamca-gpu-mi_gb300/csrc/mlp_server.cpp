@@ -296,7 +296,8 @@ static int server_step(mlp_server* s, int iters) {
         max_large = std::max(max_large, sz);
       }
     }
-    const int shape = s->shape >= 0 ? s->shape : default_shape(max_size, nact);
+    const int pick = s->shape >= 0 ? s->shape : default_shape(max_size, nact);
+    const int shape = s->wide && all_nb ? wide_shape(pick) : pick;
     size_t ntiles = 0;
     for (int q = 0; q < nact; q++) {
       const int sz = s->active[q].job->size;
@@ -319,6 +320,8 @@ static int server_step(mlp_server* s, int iters) {
     for (int it = 0; it < iters; it++) {
       if (!s->wide && all_nb)
         MLP_CUDA(launch_sweep_dvnd(s->dtiles, (int)t, s->djobs, shape, false, s->stream), "sweep kernel");
+      else if (all_nb)
+        MLP_CUDA(launch_sweep_dvnd_wide(s->dtiles, (int)t, s->djobs, shape, s->stream), "sweep kernel");
       else
         MLP_CUDA(launch_sweep(s->dtiles, (int)t, s->djobs, s->wide, shape, true, s->stream), "sweep kernel");
       if (nact >= kSoloMinJobs) {

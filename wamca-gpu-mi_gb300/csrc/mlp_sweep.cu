@@ -111,6 +111,8 @@ __global__ void __launch_bounds__(TL, CAP ? 1024 / TL : 1) k_sweep_dvnd(const Sw
       // r0 + s; else column r0 + L0 + s - TR), then the terms themselves.
       constexpr int kS = (TR + NCS + TL - 1) / TL;
       const int32_t* __restrict__ w = J->w;
+      // A 64-bit search's prefix arrays hold 64-bit words: their low halves.
+      const int ws = (J->flags & kFlagWide) ? 2 : 1;
       const uint32_t* __restrict__ Wg = (const uint32_t*)J->W;
       const uint32_t* __restrict__ Qg = (const uint32_t*)J->Q;
       const int32_t* __restrict__ Ag = J->A;
@@ -125,8 +127,8 @@ __global__ void __launch_bounds__(TL, CAP ? 1024 / TL : 1) k_sweep_dvnd(const Sw
           x.w1 = (uint32_t)w[p + 1];  // zero at and beyond sz (arrays padded to sz + 8)
           x.w2 = (uint32_t)w[p + 2];
           x.w3 = (uint32_t)w[p + 3];
-          x.W = Wg[p];
-          x.Q = Qg[p];
+          x.W = Wg[ws * p];
+          x.Q = Qg[ws * p];
           x.A1 = (uint32_t)Ag[p];
           x.A2 = (uint32_t)Ag[pad + p];
           x.A3 = (uint32_t)Ag[2 * pad + p];
