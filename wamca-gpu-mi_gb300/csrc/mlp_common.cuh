@@ -234,9 +234,13 @@ MLP_HD void conflict_interval(int id, int i, int j, int& a, int& b) {
 // i.e. [la, lb + e(t_lo)] and [ha, hb + e(t_hi)] intersect: widening every
 // move's own intervals by e of its own type on the right makes the test
 // symmetric and free of the types.  A shape packs the two right-widened
-// intervals as four 16-bit fields (a1, b1, a2, b2); a pair conflicts iff one
-// of its four interval pairs intersects.  Exhaustively equal to !canMerge
-// over every move pair of small tours (tests/shape_conflict_check.cpp).
+// intervals: a1 | a2 << 16 in its low word, b1 | b2 << 16 in its high word with
+// bits 15 and 31 set; a pair conflicts iff one of its four interval pairs
+// intersects.  Positions stay below 2^15, so a field of B | guard minus A keeps
+// its guard bit iff b >= a: two interval pairs are tested by two subtractions.
+// Exhaustively equal to !canMerge over every move pair of small tours
+// (tests/shape_conflict_check.cpp).
+constexpr uint32_t kShapeGuard = 0x80008000u;
 MLP_HD uint64_t move_shape(int id, int i, int j) {
   uint32_t a1, b1, a2, b2;
   if (id == 0) {
@@ -246,14 +250,14 @@ MLP_HD uint64_t move_shape(int id, int i, int j) {
   } else {
     a1 = a2 = (uint32_t)imin_(i, j); b1 = b2 = (uint32_t)(imax_(i, j) + id - 1);
   }
-  return (uint64_t)(a1 | (b1 << 16)) | ((uint64_t)(a2 | (b2 << 16)) << 32);
+  return (uint64_t)(a1 | (a2 << 16)) | ((uint64_t)(b1 | (b2 << 16) | kShapeGuard) << 32);
 }
+MLP_HD uint32_t swap_halves(uint32_t v) { return (v << 16) | (v >> 16); }
 MLP_HD bool shapes_conflict(uint64_t s1, uint64_t s2) {
-  const uint32_t p1 = (uint32_t)s1, p2 = (uint32_t)(s1 >> 32), q1 = (uint32_t)s2, q2 = (uint32_t)(s2 >> 32);
-  const uint32_t pa1 = p1 & 0xffffu, pb1 = p1 >> 16, pa2 = p2 & 0xffffu, pb2 = p2 >> 16;
-  const uint32_t qa1 = q1 & 0xffffu, qb1 = q1 >> 16, qa2 = q2 & 0xffffu, qb2 = q2 >> 16;
-  return (pa1 <= qb1 && qa1 <= pb1) | (pa1 <= qb2 && qa2 <= pb1) | (pa2 <= qb1 && qa1 <= pb2) |
-         (pa2 <= qb2 && qa2 <= pb2);
+  const uint32_t A = (uint32_t)s1, B = (uint32_t)(s1 >> 32), C = (uint32_t)s2, D = (uint32_t)(s2 >> 32);
+  const uint32_t same = (D - A) & (B - C);                                // (1, 1) and (2, 2)
+  const uint32_t cross = (swap_halves(D) - A) & (B - swap_halves(C));     // (1, 2) and (2, 1)
+  return ((same | cross) & kShapeGuard) != 0;
 }
 
 // ---------------- device job descriptor ----------------

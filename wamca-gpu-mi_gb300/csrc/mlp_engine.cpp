@@ -612,6 +612,7 @@ int JobSet::init() {
   }
   MLP_CUDA(configure_merge(merge_smem_ ? merge_smem_bytes(max_size_) : 0), "configure merge");
   MLP_CUDA(configure_small(), "configure search");
+  MLP_CUDA(configure_merge_one(), "configure merge");
   MLP_CUDA(cudaMallocHost(&hstats_, sizeof(int64_t) * kStatWords * jobs_.size()), "cudaMallocHost");
   MLP_CUDA(cudaMallocHost(&hstats2_, sizeof(int64_t) * kStatWords * jobs_.size()), "cudaMallocHost");
   for (int b = 0; b < 2; b++) {
@@ -830,7 +831,9 @@ int JobSet::launch_iteration() {
     const int st = launch_dvnd_sweep();
     if (st != kOk) return st;
   }
-  if (solo_merge())
+  if (merge_mode_ == kMergeAuto && merge_one_serves((int)all_jobs_.size(), max_size_))
+    MLP_CUDA(launch_merge_one(djobs_, (int)jobs_.size(), wide_, max_size_, stream_), "merge kernel");
+  else if (solo_merge())
     MLP_CUDA(launch_merge_solo(djobs_, (int)jobs_.size(), wide_, solo_smem_, max_size_, stream_), "merge kernel");
   else
     MLP_CUDA(launch_merge(djobs_, (int)jobs_.size(), wide_, merge_smem_, max_size_, stream_), "merge kernel");

@@ -162,8 +162,9 @@ class JobSet {
   JobDev* device_jobs() const { return djobs_; }
   // One DVND iteration over the current jobs (no statistics reset).
   int launch_iteration();
-  // Merge kernel: kMergeAuto (one CTA per job for sets of kSoloMinJobs jobs
-  // or more, a six-CTA cluster per job otherwise), kMergeCluster, kMergeSolo.
+  // Merge kernel: kMergeAuto (k_merge_one where merge_one_serves(); else
+  // k_merge_solo for sets of kSoloMinJobs jobs or more, a six-CTA cluster per
+  // job otherwise), kMergeCluster, kMergeSolo.
   int set_merge_mode(int mode);
   bool solo_merge() const;
   // TOTAL candidate mode: every move the sweep evaluates is a merge

@@ -81,6 +81,12 @@ cudaError_t launch_merge(const JobDev* jobs, int njobs, bool wide, bool use_smem
 // One CTA per job (throughput: sets of many jobs).  Identical results.
 cudaError_t launch_merge_solo(const JobDev* jobs, int njobs, bool wide, bool use_smem, int max_size,
                               cudaStream_t s);
+// One CTA per job with its lists in shared memory (mlp_merge_one.cu), for tours
+// of at most merge_one_max_size() positions.  Identical results.
+int merge_one_max_size();
+bool merge_one_serves(int njobs, int max_size);
+cudaError_t configure_merge_one();
+cudaError_t launch_merge_one(const JobDev* jobs, int njobs, bool wide, int max_size, cudaStream_t s);
 // TOTAL candidate mode (every evaluated move is a merge candidate).
 // The collecting sweep appends each job's improving moves to its TOTAL lists
 // (compiled for the tile shapes total_shape() picks); the TOTAL greedy selects

@@ -642,5 +642,190 @@ __device__ __forceinline__ void stage3_select(int m3, const uint64_t* key3, cons
   }
 }
 
+// The stage-3 list.
+struct MoveList {
+  uint64_t *key, *shp;
+  uint32_t* ij;
+  uint8_t* st;
+  int* count;
+  __device__ __forceinline__ void put(int s, int nb, uint64_t k, uint32_t m) const {
+    key[s] = ((k >> kCtxBits) << (kCtxBits + 3)) | ((uint64_t)nb << kCtxBits) | (k & ((1u << kCtxBits) - 1));
+    shp[s] = move_shape(nb, (int)(m & 0xffff), (int)(m >> 16));
+    ij[s] = m;
+    st[s] = kUndec;
+  }
+};
+
+// Stage 2 of the swap by the first nthreads threads (named barrier 1) for
+// c <= 32 W candidates (key, move): they are ranked by key, every tour
+// position gets the mask of the candidates with an endpoint there (pmask: W
+// zeroed words a position), and one warp settles them in rounds: a candidate is kept once no earlier one
+// within a position of its endpoints (f_canSwapMerge) is left, and leaves once
+// one is kept.
+template <int W, typename MoveOf>
+__device__ __forceinline__ void swap_greedy(int c, int nthreads, const uint64_t* lkey, MoveOf ij_of, uint64_t* skey,
+                                            uint32_t* sij, uint32_t* pmask, const MoveList& out) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int x = tid; x < c; x += nthreads) {
+    const uint64_t k = lkey[x];
+    int r = 0;
+#pragma unroll 8
+    for (int y = 0; y < c; y++) r += lkey[y] < k ? 1 : 0;
+    skey[r] = k;
+    sij[r] = ij_of(x);
+  }
+  group_sync(1, nthreads);
+  for (int x = tid; x < c; x += nthreads) {
+    const uint32_t m = sij[x], bit = 1u << lane;
+    atomicOr(&pmask[(m & 0xffff) * W + (x >> 5)], bit);
+    atomicOr(&pmask[(m >> 16) * W + (x >> 5)], bit);
+  }
+  group_sync(1, nthreads);
+  if (tid >= 32) return;
+  uint32_t row[W][W], in[W], und[W];
+  uint8_t st[W];
+#pragma unroll
+  for (int q = 0; q < W; q++) {
+    const int x = 32 * q + lane;
+    st[q] = x < c ? kUndec : kNone;
+    in[q] = und[q] = 0;
+#pragma unroll
+    for (int w = 0; w < W; w++) row[q][w] = 0;
+    if (32 * q >= c) continue;
+    if (x < c) {
+      const uint32_t m = sij[x];
+      const int i = (int)(m & 0xffff), j = (int)(m >> 16);
+#pragma unroll
+      for (int e = -1; e <= 1; e++) {
+#pragma unroll
+        for (int w = 0; w <= q; w++) row[q][w] |= pmask[(i + e) * W + w] | pmask[(j + e) * W + w];
+      }
+#pragma unroll
+      for (int w = 0; w < W; w++) row[q][w] &= w < q ? 0xffffffffu : (w == q ? (1u << lane) - 1u : 0u);
+    }
+    und[q] = __ballot_sync(kFull, st[q] == kUndec);
+  }
+  for (int round = 0; round < c; round++) {
+    uint32_t left = 0;
+#pragma unroll
+    for (int q = 0; q < W; q++) {
+      if (st[q] != kUndec) continue;
+      uint32_t hin = 0, hund = 0;
+#pragma unroll
+      for (int w = 0; w <= q; w++) {
+        hin |= row[q][w] & in[w];
+        hund |= row[q][w] & und[w];
+      }
+      if (hin) st[q] = kOut;
+      else if (!hund) st[q] = kIn;
+    }
+#pragma unroll
+    for (int q = 0; q < W; q++) {
+      if (32 * q >= c) continue;
+      in[q] = __ballot_sync(kFull, st[q] == kIn);
+      und[q] = __ballot_sync(kFull, st[q] == kUndec);
+      left |= und[q];
+    }
+    if (!left) break;
+  }
+  int total = 0;
+#pragma unroll
+  for (int q = 0; q < W; q++) total += __popc(in[q]);
+  int base = 0;
+  if (lane == 0 && total) base = atomicAdd(out.count, total);
+  base = __shfl_sync(kFull, base, 0);
+#pragma unroll
+  for (int q = 0; q < W; q++) {
+    if (in[q] == 0) continue;
+    if (st[q] == kIn) out.put(base + __popc(in[q] & ((1u << lane) - 1u)), 0, skey[32 * q + lane], sij[32 * q + lane]);
+    base += __popc(in[q]);
+  }
+}
+
+// Kept move (key, ij) enters the position map: src[p] is the old position of
+// new position p (called by a warp; kept moves change disjoint positions).
+__device__ __forceinline__ void map_positions(uint64_t key, uint32_t ij, int32_t* src) {
+  const int lane = threadIdx.x & 31, id = id_of(key);
+  const int i = (int)(ij & 0xffff), j = (int)(ij >> 16);
+  if (id == 0) {
+    if (lane < 2) src[lane ? j : i] = lane ? i : j;
+  } else {
+    int f0, f1;
+    move_footprint(id, i, j, f0, f1);
+    for (int p = f0 + lane; p <= f1; p += 32) src[p] = move_source(id, i, j, p);
+  }
+}
+
+// Stage 3 of at most 32 * W moves by the whole CTA: every warp computes a
+// share of the conflict rows (bit y of row x: y precedes x and cannot be
+// merged with it), one warp settles all moves in rounds of ballots (the other
+// warps' issue slots stay free), and every warp maps the positions of its share
+// of the kept ones.  Returns the number of kept moves.
+template <int W>
+__device__ __forceinline__ int stage3_warps(int m3, const MoveList& list, uint32_t* bits, int32_t* src) {
+  __shared__ uint32_t s_kept[4];
+  static_assert(W <= 4, "kept words");
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int x = wid; x < m3; x += nw) {
+    const uint64_t kx = list.key[x], sx = list.shp[x];
+#pragma unroll
+    for (int w = 0; w < W; w++) {
+      if (32 * w >= m3) break;
+      const int y = 32 * w + lane;
+      const uint32_t word = __ballot_sync(kFull, y < m3 && list.key[y] < kx && shapes_conflict(list.shp[y], sx));
+      if (lane == 0) bits[x * W + w] = word;
+    }
+  }
+  __syncthreads();
+  if (wid == 0) {
+    uint32_t row[W][W], in[W], und[W];
+    bool undec[W];
+#pragma unroll
+    for (int q = 0; q < W; q++) {
+      const int x = 32 * q + lane;
+      undec[q] = x < m3;
+#pragma unroll
+      for (int w = 0; w < W; w++) row[q][w] = x < m3 && 32 * w < m3 ? bits[x * W + w] : 0u;
+      in[q] = 0u;
+      und[q] = __ballot_sync(kFull, undec[q]);
+    }
+    for (int round = 0; round < m3; round++) {
+      uint32_t left = 0, now[W];
+#pragma unroll
+      for (int q = 0; q < W; q++) {
+        now[q] = 0u;
+        if (und[q] == 0) continue;
+        uint32_t hin = 0, hund = 0;
+#pragma unroll
+        for (int w = 0; w < W; w++) {
+          hin |= row[q][w] & in[w];
+          hund |= row[q][w] & und[w];
+        }
+        now[q] = __ballot_sync(kFull, undec[q] && !hin && !hund);  // joins
+        undec[q] = undec[q] && !hin && hund;
+      }
+#pragma unroll
+      for (int q = 0; q < W; q++) {
+        if (und[q] == 0) continue;
+        in[q] |= now[q];
+        und[q] = __ballot_sync(kFull, undec[q]);
+        left |= und[q];
+      }
+      if (!left) break;
+    }
+    if (lane == 0) {
+#pragma unroll
+      for (int q = 0; q < W; q++) s_kept[q] = in[q];
+    }
+  }
+  __syncthreads();
+  int kept = 0;
+#pragma unroll
+  for (int q = 0; q < W; q++) kept += __popc(s_kept[q]);
+  for (int x = wid; x < m3; x += nw)
+    if ((s_kept[x >> 5] >> (x & 31)) & 1u) map_positions(list.key[x], list.ij[x], src);
+  return kept;
+}
+
 }  // namespace
 }  // namespace mlp

@@ -9,10 +9,9 @@
 //      is built on the device from the coordinates, the start tour is uploaded
 //      and the ADS prefix arrays are prepared, with no host synchronisation;
 //   2. runs `iters` DVND iterations over every admitted search in shared
-//      launches: one sweep over all searches' tiles, then one merge launch for
-//      the searches whose merge fits shared memory and one for the rest (one
-//      CTA per search when many are active, a six-CTA cluster per search
-//      otherwise).  A search that converged or used its sweep limit turns
+//      launches: one sweep over all searches' tiles, then one merge launch (one
+//      CTA per search); with a search too large for that merge, one launch for
+//      the searches whose merge fits shared memory and one for the rest.  A search that converged or used its sweep limit turns
 //      into no-op CTAs;
 //   3. reads every slot's statistics (one copy) and retires the finished
 //      searches: tour and statistics become the request's result, the memory
@@ -324,7 +323,9 @@ static int server_step(mlp_server* s, int iters) {
         MLP_CUDA(launch_sweep_dvnd_wide(s->dtiles, (int)t, s->djobs, shape, s->stream), "sweep kernel");
       else
         MLP_CUDA(launch_sweep(s->dtiles, (int)t, s->djobs, s->wide, shape, true, s->stream), "sweep kernel");
-      if (nact >= kSoloMinJobs) {
+      if (merge_one_serves(nact, max_size)) {
+        MLP_CUDA(launch_merge_one(s->djobs, nact, s->wide, max_size, s->stream), "merge kernel");
+      } else if (nact >= kSoloMinJobs) {
         MLP_CUDA(launch_merge_solo(s->djobs, ksmall, s->wide, true, max_small, s->stream), "merge kernel");
         MLP_CUDA(launch_merge_solo(s->djobs + ksmall, nact - ksmall, s->wide, false, max_large, s->stream),
                  "merge kernel");
@@ -440,6 +441,7 @@ MLP_API int mlp_server_create(int64_t memory_budget, int32_t wide, int32_t max_a
   for (int q = max_active - 1; q >= 0; q--) s->free_slots.push_back(q);
   MLP_CUDA(configure_prepare(), "configure prepare kernel");
   MLP_CUDA(configure_merge(merge_smem_bytes(merge_smem_max_size())), "configure merge");
+  MLP_CUDA(configure_merge_one(), "configure merge");
   *out = s.release();
   return kOk;
 }

@@ -219,27 +219,13 @@ __device__ __forceinline__ void small_tile(uint64_t* keys, int sz, int n, int rs
 // Gathering steps of one neighbourhood's candidates.
 constexpr int kGather = (kSmallMaxSize + 32 * kIntervalWarps - 1) / (32 * kIntervalWarps);
 
-// The stage-3 list.
-struct SmallList {
-  uint64_t *key, *shp;
-  uint32_t* ij;
-  uint8_t* st;
-  int* count;
-  __device__ __forceinline__ void put(int s, int nb, uint64_t k, uint32_t m) const {
-    key[s] = ((k >> kCtxBits) << (kCtxBits + 3)) | ((uint64_t)nb << kCtxBits) | (k & ((1u << kCtxBits) - 1));
-    shp[s] = move_shape(nb, (int)(m & 0xffff), (int)(m >> 16));
-    ij[s] = m;
-    st[s] = kUndec;
-  }
-};
-
 // Stage 2 of 2-opt or Or-opt-k by one warp: of its c candidates the one of the
 // smallest (delta, block) is kept and those whose conflict interval meets its
 // own leave, repeatedly (the greedy in that order; few are kept).  A lane's
 // candidates are words delta | block, interval.
 template <int PER>
 __device__ __forceinline__ void small_intervals(int nb, int c, const uint64_t* lkey, const uint32_t* lij,
-                                                const SmallList& out) {
+                                                const MoveList& out) {
   const int lane = threadIdx.x & 31;
   uint32_t hi[PER], lo[PER];
   constexpr uint32_t kDead = 0xffffffffu;
@@ -282,168 +268,6 @@ __device__ __forceinline__ void small_intervals(int nb, int c, const uint64_t* l
 #pragma unroll
   for (int q = 0; q < PER; q++)
     if ((kept >> q) & 1u) out.put(atomicAdd(out.count, 1), nb, lkey[32 * q + lane], lij[32 * q + lane]);
-}
-
-// Stage 2 of the swap by its warps: the candidates are ranked by key, every
-// tour position gets the mask of the candidates with an endpoint there, and
-// one warp settles them in rounds: a candidate is kept once no earlier one
-// within a position of its endpoints (f_canSwapMerge) is left, and leaves once
-// one is kept.
-template <int W>
-__device__ __forceinline__ void small_swaps(int c, int sz, const uint64_t* lkey, const uint32_t* lij, uint64_t* skey,
-                                            uint32_t* sij, uint32_t* pmask, const SmallList& out) {
-  constexpr int kThreads = 32 * kSwapWarps;
-  const int tid = threadIdx.x, lane = tid & 31;
-  for (int x = tid; x < c; x += kThreads) {
-    const uint64_t k = lkey[x];
-    int r = 0;
-#pragma unroll 8
-    for (int y = 0; y < c; y++) r += lkey[y] < k ? 1 : 0;
-    skey[r] = k;
-    sij[r] = lij[x];
-  }
-  group_sync(1, kThreads);
-  for (int x = tid; x < c; x += kThreads) {
-    const uint32_t m = sij[x], bit = 1u << lane;
-    atomicOr(&pmask[(m & 0xffff) * W + (x >> 5)], bit);
-    atomicOr(&pmask[(m >> 16) * W + (x >> 5)], bit);
-  }
-  group_sync(1, kThreads);
-  if (tid >= 32) return;
-  uint32_t row[W][W], in[W], und[W];
-  uint8_t st[W];
-#pragma unroll
-  for (int q = 0; q < W; q++) {
-    const int x = 32 * q + lane;
-    st[q] = x < c ? kUndec : kNone;
-    in[q] = und[q] = 0;
-#pragma unroll
-    for (int w = 0; w < W; w++) row[q][w] = 0;
-    if (32 * q >= c) continue;
-    if (x < c) {
-      const uint32_t m = sij[x];
-      const int i = (int)(m & 0xffff), j = (int)(m >> 16);
-#pragma unroll
-      for (int e = -1; e <= 1; e++) {
-#pragma unroll
-        for (int w = 0; w <= q; w++) row[q][w] |= pmask[(i + e) * W + w] | pmask[(j + e) * W + w];
-      }
-#pragma unroll
-      for (int w = 0; w < W; w++) row[q][w] &= w < q ? 0xffffffffu : (w == q ? (1u << lane) - 1u : 0u);
-    }
-    und[q] = __ballot_sync(kFull, st[q] == kUndec);
-  }
-  for (int round = 0; round < c; round++) {
-    uint32_t left = 0;
-#pragma unroll
-    for (int q = 0; q < W; q++) {
-      if (st[q] != kUndec) continue;
-      uint32_t hin = 0, hund = 0;
-#pragma unroll
-      for (int w = 0; w <= q; w++) {
-        hin |= row[q][w] & in[w];
-        hund |= row[q][w] & und[w];
-      }
-      if (hin) st[q] = kOut;
-      else if (!hund) st[q] = kIn;
-    }
-#pragma unroll
-    for (int q = 0; q < W; q++) {
-      if (32 * q >= c) continue;
-      in[q] = __ballot_sync(kFull, st[q] == kIn);
-      und[q] = __ballot_sync(kFull, st[q] == kUndec);
-      left |= und[q];
-    }
-    if (!left) break;
-  }
-  int total = 0;
-#pragma unroll
-  for (int q = 0; q < W; q++) total += __popc(in[q]);
-  int base = 0;
-  if (lane == 0 && total) base = atomicAdd(out.count, total);
-  base = __shfl_sync(kFull, base, 0);
-#pragma unroll
-  for (int q = 0; q < W; q++) {
-    if (in[q] == 0) continue;
-    if (st[q] == kIn) out.put(base + __popc(in[q] & ((1u << lane) - 1u)), 0, skey[32 * q + lane], sij[32 * q + lane]);
-    base += __popc(in[q]);
-  }
-}
-
-// Kept move (key, ij) enters the position map: src[p] is the old position of
-// new position p (called by a warp; kept moves change disjoint positions).
-__device__ __forceinline__ void small_map(uint64_t key, uint32_t ij, int32_t* src) {
-  const int lane = threadIdx.x & 31, id = id_of(key);
-  const int i = (int)(ij & 0xffff), j = (int)(ij >> 16);
-  if (id == 0) {
-    if (lane < 2) src[lane ? j : i] = lane ? i : j;
-  } else {
-    int f0, f1;
-    move_footprint(id, i, j, f0, f1);
-    for (int p = f0 + lane; p <= f1; p += 32) src[p] = move_source(id, i, j, p);
-  }
-}
-
-// Stage 3 of at most 32 * W moves by the whole CTA: every warp computes a
-// share of the conflict rows (bit y of row x: y precedes x and cannot be
-// merged with it), then every warp settles all moves by itself in rounds of
-// ballots and maps the positions of its share of the kept ones.  Returns the
-// number of kept moves.
-template <int W>
-__device__ __forceinline__ int small_stage3(int m3, const SmallList& list, uint32_t* bits, int32_t* src) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int x = wid; x < m3; x += nw) {
-    const uint64_t kx = list.key[x], sx = list.shp[x];
-#pragma unroll
-    for (int w = 0; w < W; w++) {
-      const int y = 32 * w + lane;
-      const uint32_t word = __ballot_sync(kFull, y < m3 && list.key[y] < kx && shapes_conflict(list.shp[y], sx));
-      if (lane == 0) bits[x * W + w] = word;
-    }
-  }
-  __syncthreads();
-  uint32_t row[W][W], in[W], und[W];
-  bool undec[W];
-#pragma unroll
-  for (int q = 0; q < W; q++) {
-    const int x = 32 * q + lane;
-    undec[q] = x < m3;
-#pragma unroll
-    for (int w = 0; w < W; w++) row[q][w] = x < m3 ? bits[x * W + w] : 0u;
-    in[q] = 0u;
-    und[q] = __ballot_sync(kFull, undec[q]);
-  }
-  for (int round = 0; round < m3; round++) {
-    uint32_t left = 0, now[W];
-#pragma unroll
-    for (int q = 0; q < W; q++) {
-      uint32_t hin = 0, hund = 0;
-#pragma unroll
-      for (int w = 0; w < W; w++) {
-        hin |= row[q][w] & in[w];
-        hund |= row[q][w] & und[w];
-      }
-      now[q] = __ballot_sync(kFull, undec[q] && !hin && !hund);  // joins
-      undec[q] = undec[q] && !hin && hund;
-    }
-#pragma unroll
-    for (int q = 0; q < W; q++) {
-      in[q] |= now[q];
-      und[q] = __ballot_sync(kFull, undec[q]);
-      left |= und[q];
-    }
-    if (!left) break;
-  }
-  int kept = 0;
-#pragma unroll
-  for (int q = 0; q < W; q++) kept += __popc(in[q]);
-  for (int x = wid; x < m3; x += nw) {
-    uint32_t word = in[0];
-#pragma unroll
-    for (int q = 1; q < W; q++) word = (x >> 5) == q ? in[q] : word;
-    if ((word >> (x & 31)) & 1u) small_map(list.key[x], list.ij[x], src);
-  }
-  return kept;
 }
 
 // One search to its local optimum (or `limit` sweeps), by one cluster.
@@ -587,7 +411,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __re
     cluster.sync();  // the keys, for the merging CTA
     if (merger) {
       // ---- stage 2: the candidates of each neighbourhood ----
-      const SmallList list{reinterpret_cast<uint64_t*>(smem + lay.key3), reinterpret_cast<uint64_t*>(smem + lay.shp3),
+      const MoveList list{reinterpret_cast<uint64_t*>(smem + lay.key3), reinterpret_cast<uint64_t*>(smem + lay.shp3),
                            reinterpret_cast<uint32_t*>(smem + lay.ij3), smem + lay.st3, &s_m3};
       {
         const int nb = wid < kSwapWarps ? 0 : 1 + (wid - kSwapWarps) / kIntervalWarps;
@@ -629,9 +453,10 @@ __global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __re
         if (nb == 0) {
           uint64_t* skey = reinterpret_cast<uint64_t*>(smem + lay.skey);
           uint32_t* sij = reinterpret_cast<uint32_t*>(smem + lay.sij);
-          if (c <= 32) small_swaps<1>(c, sz, lkey, lij, skey, sij, pmask, list);
-          else if (c <= 128) small_swaps<4>(c, sz, lkey, lij, skey, sij, pmask, list);
-          else small_swaps<kSmallWords>(c, sz, lkey, lij, skey, sij, pmask, list);
+          auto ij_of = [&](int x) { return lij[x]; };
+          if (c <= 32) swap_greedy<1>(c, gnt, lkey, ij_of, skey, sij, pmask, list);
+          else if (c <= 128) swap_greedy<4>(c, gnt, lkey, ij_of, skey, sij, pmask, list);
+          else swap_greedy<kSmallWords>(c, gnt, lkey, ij_of, skey, sij, pmask, list);
         } else if (gtid < 32) {
           if (c <= 32) small_intervals<1>(nb, c, lkey, lij, list);
           else if (c <= 128) small_intervals<4>(nb, c, lkey, lij, list);
@@ -644,15 +469,15 @@ __global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __re
       uint32_t* bits = reinterpret_cast<uint32_t*>(smem + lay.bits);
       int kept;
       if (m3 <= 32) {
-        kept = small_stage3<1>(m3, list, bits, src);
+        kept = stage3_warps<1>(m3, list, bits, src);
       } else if (m3 <= 128) {
-        kept = small_stage3<4>(m3, list, bits, src);
+        kept = stage3_warps<4>(m3, list, bits, src);
       } else {
         if (tid == 0) s_ns = 0;
         stage3_select(m3, list.key, list.shp, list.st, bits);
         for (int x = wid; x < m3; x += nw) {
           if (list.st[x] != kIn) continue;
-          small_map(list.key[x], list.ij[x], src);
+          map_positions(list.key[x], list.ij[x], src);
           if (lane == 0) atomicAdd(&s_ns, 1);
         }
         kept = -1;
