@@ -1,0 +1,53 @@
+"""Results read by one kernel into pinned memory (batch results, recorded
+passes) and searches of a few iterations launched without the device-side loop,
+against the oracle at the edges of their copies and of the rule."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,seed", [(5, 1), (511, 2), (513, 3)])
+@pytest.mark.parametrize("wide", [False, True])
+def test_recorded_pass_by_capacity(mlpgpu_mod, n, seed, wide):
+    """The first min(moves, capacity) moves, none of a later one's left over."""
+    x, y = oracle.clustered_instance(n, seed)
+    t, D = oracle.random_perm_tour(n, seed), oracle.dist(x, y, True)
+    s = mlpgpu_mod.Solver(mlpgpu_mod.Problem.from_coords(x, y), wide=wide)
+    for nb in range(5):
+        want_tour, want_cost, want = oracle.pass_(nb, t, D, wide)
+        for cap in (1 << 15, 1, 3, 0):
+            s.set_tour(t)
+            cost, moves = s.pass_(nb, max_moves=cap)
+            assert cost == want_cost and moves == want[:cap]
+            assert np.array_equal(s.tour(), want_tour)
+
+
+@pytest.mark.parametrize("n", [5, 100, 420])
+@pytest.mark.parametrize("iters", [1, 7, 8, 9])
+def test_few_iterations(mlpgpu_mod, n, iters):
+    """Either side of the limit below which the iterations are launched as such."""
+    x, y = oracle.uniform_instance(n, n)
+    t = oracle.random_perm_tour(n, n)
+    s = mlpgpu_mod.Solver(mlpgpu_mod.Problem.from_coords(x, y))
+    s.set_tour(t)
+    st = s.dvnd(max_iters=iters)
+    want_tour, want = oracle.dvnd(t, oracle.dist(x, y, True), False, max_iters=iters)
+    assert np.array_equal(s.tour(), want_tour)
+    assert all(st[k] == want[k] for k in ("cost", "iterations", "moves", "evals"))
+
+
+def test_batch_results_in_any_order(mlpgpu_mod):
+    sizes = [5, 6, 511, 512, 40]
+    b, want = mlpgpu_mod.Batch(), []
+    for q, n in enumerate(sizes):
+        x, y = oracle.clustered_instance(n, q)
+        t = oracle.random_perm_tour(n, q)
+        b.add(mlpgpu_mod.Problem.from_coords(x, y), t)
+        want.append(oracle.dvnd(t, oracle.dist(x, y, True)))
+    b.run()
+    for q in (2, 0, 4, 3, 1, 2):
+        t, st = b.result(q)
+        assert np.array_equal(t, want[q][0]) and st["cost"] == want[q][1]["cost"]

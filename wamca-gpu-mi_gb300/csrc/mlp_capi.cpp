@@ -563,34 +563,22 @@ MLP_API int mlp_solver_pass(mlp_solver_t s, int32_t nb, int32_t max_moves, int32
   if (max_moves > 0 && (!ids || !is || !js || !costs)) return arg_error("null move arrays");
   MLP_TRY(s->set->set_mask(1 << nb));
   MLP_TRY(s->set->set_record_moves(true));
-  const int rs = s->set->run(1, true);
+  const int rs = s->set->run(1, !s->set->loops_on_device());
   MLP_TRY(s->set->set_record_moves(false));
   MLP_TRY(rs);
-  mlp_dvnd_stats_t st;
-  std::vector<std::array<int64_t, kStatWords>> raw;
-  MLP_TRY(s->set->read_stats(&raw));
-  MLP_TRY(solver_stats(s, &st, 1 << nb));
-  const int applied = (int)raw[0][kStatLastMoves];
-  const int take = std::min(std::min(applied, (int)std::max(0, max_moves)), s->job->moves_cap);
-  if (take > 0) {
-    std::vector<uint32_t> mv(take);
-    std::vector<int64_t> mc(take);
-    MLP_CUDA(cudaMemcpyAsync(mv.data(), s->job->dev.moves_out, 4 * take, cudaMemcpyDeviceToHost,
-                             s->set->stream()),
-             "copy moves");
-    MLP_CUDA(cudaMemcpyAsync(mc.data(), s->job->dev.moves_cost, 8 * take, cudaMemcpyDeviceToHost,
-                             s->set->stream()),
-             "copy moves");
-    MLP_CUDA(cudaStreamSynchronize(s->set->stream()), "sync");
-    for (int q = 0; q < take; q++) {
-      ids[q] = (int32_t)(mv[q] & 0xf);
-      is[q] = (int32_t)((mv[q] >> 4) & 0x3fff);
-      js[q] = (int32_t)(mv[q] >> 18);
-      costs[q] = mc[q];
-    }
+  const int cap = std::min(std::max(0, (int)max_moves), s->job->moves_cap);
+  const int64_t *st, *mc;
+  const uint32_t* mv;
+  MLP_TRY(s->set->read_pass(cap, &st, &mc, &mv));
+  const int applied = (int)st[kStatLastMoves], take = std::min(applied, cap);
+  for (int q = 0; q < take; q++) {
+    ids[q] = (int32_t)(mv[q] & 0xf);
+    is[q] = (int32_t)((mv[q] >> 4) & 0x3fff);
+    js[q] = (int32_t)(mv[q] >> 18);
+    costs[q] = mc[q];
   }
   if (count) *count = applied;
-  if (new_cost) *new_cost = st.cost;
+  if (new_cost) *new_cost = st[kStatCost];
   return kOk;
 }
 
@@ -598,7 +586,7 @@ MLP_API int mlp_solver_dvnd(mlp_solver_t s, int32_t nb_mask, int32_t max_iters, 
   MLP_RANGE("mlp_solver_dvnd");
   if (!s) return arg_error("null solver");
   MLP_TRY(s->set->set_mask(nb_mask));
-  MLP_TRY(s->set->run(max_iters, true));
+  MLP_TRY(s->set->run(max_iters, !s->set->loops_on_device()));  // the statistics' read waits
   return solver_stats(s, stats, nb_mask);
 }
 
@@ -917,21 +905,22 @@ MLP_API int mlp_batch_result(mlp_batch_t b, int32_t job, int32_t* tour, int32_t 
   Job* j = b->jobs[job].get();
   if (tour) {
     if (len < j->size) return arg_error("buffer shorter than size");
-    MLP_CUDA(cudaMemcpyAsync(tour, j->dev.tour, sizeof(int32_t) * j->size, cudaMemcpyDeviceToHost, b->stream),
-             "copy tour");
   }
+  const int64_t* st;
+  const int32_t* t;
+  const int status = b->set->read_result(job, tour != nullptr, &st, &t);
+  if (status == kErrCuda) return status;
+  if (tour) std::memcpy(tour, t, sizeof(int32_t) * j->size);
   if (stats) {
-    std::vector<std::array<int64_t, kStatWords>> st;
-    MLP_TRY(b->set->read_stats(&st));
+    MLP_TRY(status);
     std::memset(stats, 0, sizeof(*stats));
-    stats->cost = st[job][kStatCost];
-    stats->iterations = st[job][kStatIters];
-    stats->sweeps = st[job][kStatSweeps];
-    stats->moves = st[job][kStatMoves];
-    stats->evals = st[job][kStatSweeps] * b->set->evals_per_sweep(job, b->mask);
-    stats->converged = (int32_t)st[job][kStatConverged];
+    stats->cost = st[kStatCost];
+    stats->iterations = st[kStatIters];
+    stats->sweeps = st[kStatSweeps];
+    stats->moves = st[kStatMoves];
+    stats->evals = st[kStatSweeps] * b->set->evals_per_sweep(job, b->mask);
+    stats->converged = (int32_t)st[kStatConverged];
   }
-  MLP_CUDA(cudaStreamSynchronize(b->stream), "sync");
   return kOk;
 }
 

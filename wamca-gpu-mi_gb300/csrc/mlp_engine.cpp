@@ -613,7 +613,10 @@ int JobSet::init() {
   MLP_CUDA(configure_merge(merge_smem_ ? merge_smem_bytes(max_size_) : 0), "configure merge");
   MLP_CUDA(configure_small(), "configure search");
   MLP_CUDA(configure_merge_one(), "configure merge");
-  MLP_CUDA(cudaMallocHost(&hstats_, sizeof(int64_t) * kStatWords * jobs_.size()), "cudaMallocHost");
+  size_t result = kResultHead + ((size_t)max_size_ + 1) / 2;
+  for (const Job* j : jobs_) result = std::max(result, kStatWords + (size_t)j->moves_cap + ((size_t)j->moves_cap + 1) / 2);
+  MLP_CUDA(cudaMallocHost(&hstats_, sizeof(int64_t) * (kStatWords * jobs_.size() + result)), "cudaMallocHost");
+  hresult_ = hstats_ + kStatWords * jobs_.size();
   MLP_CUDA(cudaMallocHost(&hstats2_, sizeof(int64_t) * kStatWords * jobs_.size()), "cudaMallocHost");
   for (int b = 0; b < 2; b++) {
     MLP_CUDA(cudaEventCreateWithFlags(&stats_ev_[b], cudaEventDisableTiming), "event");
@@ -748,17 +751,27 @@ int JobSet::set_mask(int mask) {
     int st = ensure_all_active();
     if (st != kOk) return st;
   }
+  {
+    const int st = refuse_capture("set mask");
+    if (st != kOk) return st;
+  }
   const bool was_dvnd = dvnd_sweep();
   mask_ = mask;
   if (dvnd_sweep() != was_dvnd) drop_graphs();  // the captured sweep kernel changes
-  for (size_t q = 0; q < jobs_.size(); q++) {
-    jobs_[q]->dev.nb_mask = mask;
-    MLP_CUDA(cudaMemcpyAsync(&djobs_[q].nb_mask, &jobs_[q]->dev.nb_mask, sizeof(int32_t),
-                             cudaMemcpyHostToDevice, stream_),
-             "set mask");
-  }
-  MLP_CUDA(cudaStreamSynchronize(stream_), "set mask");
+  for (Job* j : jobs_) j->dev.nb_mask = mask;
+  // In the stream, without a wait: as one copy a job and a wait for each change,
+  // these fields took a third of a neighbourhood pass (n = 100: 142 us, now 50
+  // with its results read by one kernel; n = 1000: 190, now 62).
+  MLP_CUDA(launch_set_fields(djobs_, (int)jobs_.size(), mask, 0, 0, stream_), "set mask");
   return kOk;
+}
+
+// Host state that follows the device's must not be changed by a call that is
+// only recorded into a graph.
+int JobSet::refuse_capture(const char* what) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  MLP_CUDA(cudaStreamIsCapturing(stream_, &cs), what);
+  return cs == cudaStreamCaptureStatusNone ? kOk : cuda_status(cudaErrorStreamCaptureUnsupported, what);
 }
 
 int JobSet::set_record_moves(bool on) {
@@ -766,16 +779,14 @@ int JobSet::set_record_moves(bool on) {
     int st = ensure_all_active();
     if (st != kOk) return st;
   }
-  for (size_t q = 0; q < jobs_.size(); q++) {
-    int32_t f = jobs_[q]->dev.flags;
-    f = on ? (f | kFlagRecordMoves) : (f & ~kFlagRecordMoves);
-    if (f == jobs_[q]->dev.flags) continue;
-    jobs_[q]->dev.flags = f;
-    MLP_CUDA(cudaMemcpyAsync(&djobs_[q].flags, &jobs_[q]->dev.flags, sizeof(int32_t), cudaMemcpyHostToDevice,
-                             stream_),
-             "set flags");
+  {
+    const int st = refuse_capture("set flags");
+    if (st != kOk) return st;
   }
-  MLP_CUDA(cudaStreamSynchronize(stream_), "set flags");
+  for (Job* j : jobs_) j->dev.flags = on ? (j->dev.flags | kFlagRecordMoves) : (j->dev.flags & ~kFlagRecordMoves);
+  MLP_CUDA(launch_set_fields(djobs_, (int)jobs_.size(), mask_, on ? kFlagRecordMoves : 0, on ? 0 : kFlagRecordMoves,
+                             stream_),
+           "set flags");
   return kOk;
 }
 
@@ -954,6 +965,12 @@ int JobSet::enqueue_iterations(int iters) {
 // condition kernel runs once per pass, and a search that converges within a
 // pass leaves the rest of it as kernels that return at once.
 constexpr int kDeviceLoopBody = 16;
+// A search of at most half a body's iterations is launched as such: the loop
+// would run its whole body, the rest as launches that return at once (one
+// iteration from a random tour, n = 400: 81 us as a loop, 41 as launches; n = 1000:
+// 127 and 54; four iterations: 212 and 150; converged tours, n = 1000: 102 for any
+// limit, 38 for four).  Near the body's length both cost the same.
+constexpr int kDirectIters = kDeviceLoopBody / 2;
 
 // Every delta of the search fits 32 bits: costs are below dmax * size^2 / 2,
 // so a 64-bit job's deltas are the 32-bit ones, exactly.
@@ -983,6 +1000,10 @@ int JobSet::enqueue_device_loop(int max_iters) {
     set_error("the device-side loop needs a non-default stream");
     return kErrState;
   }
+  {
+    const int st = refuse_capture("the device-side loop");
+    if (st != kOk) return st;
+  }
   if (small_search()) {
     MLP_CUDA(launch_dvnd_small(djobs_, max_size_, wide_, max_iters, stream_), "search kernel");
     return kOk;
@@ -991,6 +1012,14 @@ int JobSet::enqueue_device_loop(int max_iters) {
   {
     const int st = ensure_tiles(dvnd_list());
     if (st != kOk) return st;
+  }
+  if (max_iters <= kDirectIters) {
+    MLP_CUDA(launch_stats_begin(djobs_, (int)jobs_.size(), max_iters, stream_), "stats kernel");
+    for (int q = 0; q < max_iters; q++) {
+      const int st = launch_iteration();
+      if (st != kOk) return st;
+    }
+    return kOk;
   }
   if (!loop_graph_ || loop_unroll_ != unroll) {
     if (loop_graph_) cudaGraphExecDestroy(loop_graph_);
@@ -1054,7 +1083,7 @@ int JobSet::run(int max_iters, bool sync) {
     int st = ensure_all_active();
     if (st != kOk) return st;
   }
-  if (device_loop_ && stream_ != 0 && all_jobs_.size() == 1) {
+  if (loops_on_device()) {
     int st = enqueue_device_loop(max_iters);
     if (st != kOk || !sync) return st;
     std::vector<std::array<int64_t, kStatWords>> s;
@@ -1153,9 +1182,33 @@ int JobSet::read_stats(std::vector<std::array<int64_t, kStatWords>>* out) {
   return check_stats(hstats_);
 }
 
+int JobSet::read_result(int job, bool tour, const int64_t** stats, const int32_t** out) {
+  const Job* j = all_jobs_[job];
+  MLP_CUDA(launch_result(dstats_, (int)all_jobs_.size(), job, tour ? j->dev.tour : nullptr, j->size, hresult_, stream_),
+           "read result");
+  MLP_CUDA(cudaStreamSynchronize(stream_), "read result");
+  *stats = hresult_;
+  *out = reinterpret_cast<const int32_t*>(hresult_ + kResultHead);
+  return check_error(hresult_[kStatWords]);
+}
+
+int JobSet::read_pass(int cap, const int64_t** stats, const int64_t** costs, const uint32_t** moves) {
+  const Job* j = all_jobs_[0];
+  MLP_CUDA(launch_pass_result(dstats_, j->dev.moves_out, j->dev.moves_cost, cap, hresult_, stream_), "read moves");
+  MLP_CUDA(cudaStreamSynchronize(stream_), "read moves");
+  *stats = hresult_;
+  *costs = hresult_ + kStatWords;
+  *moves = reinterpret_cast<const uint32_t*>(hresult_ + kStatWords + cap);
+  return check_error(hresult_[kStatError]);
+}
+
 int JobSet::check_stats(const int64_t* hst) {
   int64_t err = 0;
   for (size_t q = 0; q < all_jobs_.size(); q++) err |= hst[q * kStatWords + kStatError];
+  return check_error(err);
+}
+
+int JobSet::check_error(int64_t err) {
   if (err) {
     static const char* what[] = {"", "", "merge stage-2 hand-off timed out (no longer produced)", "kept-move region overflow",
                                  "TOTAL list overflow", "TOTAL selection invariant broken",

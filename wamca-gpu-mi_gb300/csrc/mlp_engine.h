@@ -150,6 +150,13 @@ class JobSet {
   // synchronisation.  Read the results with read_stats().
   int enqueue_device_loop(int max_iters);
   int read_stats(std::vector<std::array<int64_t, kStatWords>>* out);
+  // Waits for the stream and returns one job's statistics and, on request, its
+  // tour, or a recorded pass's first `cap` moves, in pinned memory that holds
+  // until the next of these calls.
+  int read_result(int job, bool tour, const int64_t** stats, const int32_t** out);
+  int read_pass(int cap, const int64_t** stats, const int64_t** costs, const uint32_t** moves);
+  // run() is one device-side loop, which needs no wait between its iterations.
+  bool loops_on_device() const { return device_loop_ && stream_ != 0 && all_jobs_.size() == 1; }
   int64_t evals_per_sweep(int job, int mask) const;
   const std::vector<Job*>& jobs() const { return all_jobs_; }
   // Launch only the listed jobs (indices into jobs()); converged jobs are
@@ -191,6 +198,8 @@ class JobSet {
   int ensure_tiles(int list, int buf = 0, bool sync = true);
   int dvnd_list() const { return sweep64() && !total_ ? 1 : 0; }  // the list of an iteration's sweep
   void drop_tiles() { lists_[0].ok = lists_[1].ok = false; }
+  int check_error(int64_t err);
+  int refuse_capture(const char* what);
   int check_stats(const int64_t* hst);  // the statistics' internal error words
   void drop_graphs();
   // DVND iterations evaluate all five neighbourhoods from row and column terms:
@@ -224,6 +233,7 @@ class JobSet {
   JobDev* djobs_ = nullptr;
   TileList lists_[2];
   int64_t* hstats_ = nullptr;  // pinned, kStatWords per job
+  int64_t* hresult_ = nullptr;  // behind it: room for one job's results
   int64_t* hstats2_ = nullptr;  // a second one (the batch loop reads one while the other fills)
   cudaEvent_t stats_ev_[2] = {nullptr, nullptr};
   JobDev* hjobs_[2] = {nullptr, nullptr};      // pinned staging of the job descriptors

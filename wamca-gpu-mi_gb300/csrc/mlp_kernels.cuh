@@ -69,6 +69,18 @@ cudaError_t launch_loop_condition(const JobDev* jobs, int njobs, cudaGraphCondit
 cudaError_t configure_prepare();
 // Zero the run counters of every job and set its sweep limit.
 cudaError_t launch_stats_begin(const JobDev* jobs, int njobs, int64_t limit, cudaStream_t s);
+// Neighbourhood mask and flags of every job, ordered in the stream.
+cudaError_t launch_set_fields(JobDev* jobs, int njobs, int nb_mask, int flags_on, int flags_off, cudaStream_t s);
+// One job's results into mapped pinned memory, for a caller that waits for the
+// stream: statistics (kStatWords words), the OR of all jobs' error words, then
+// (tour != null) the tour's `size` entries.
+constexpr int kResultHead = kStatWords + 2;  // words before the tour
+cudaError_t launch_result(const int64_t* stats, int njobs, int job, const int32_t* tour, int size, int64_t* out,
+                          cudaStream_t s);
+// The same after a recorded pass: statistics, then the first min(moves, cap)
+// moves: cap 64-bit costs, cap 32-bit moves.
+cudaError_t launch_pass_result(const int64_t* stats, const uint32_t* moves, const int64_t* costs, int cap, int64_t* out,
+                               cudaStream_t s);
 cudaError_t launch_prepare(const JobDev* jobs, int njobs, bool wide, bool reset_stats,
                            cudaStream_t s);
 // improve_only: publish only improving candidates (DVND iterations; the
