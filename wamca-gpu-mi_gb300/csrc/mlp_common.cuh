@@ -313,6 +313,10 @@ struct JobDev {
 // 9 V_2, 10 V_3, 11 zero.  The sweep's deltas from them are given where it
 // evaluates them (k_sweep_dvnd).
 constexpr int kTermWords = 12;
+// Column terms of the moves that a column has not (past the tour's end): large,
+// so that a look at a row's signs does not take their deltas for improving
+// ones.  Only speed depends on it: every move's validity is checked.
+constexpr int32_t kTermNever = 0x40000000;
 
 #ifdef __CUDACC__
 // Programmatic dependent launch.  A kernel launched with programmatic stream
@@ -349,6 +353,9 @@ __device__ __forceinline__ void col_terms(const TermIn& x, int p, int sz, int4& 
                  (int)((sp - 2u) * (x.A2 - x.w2) + RB0 + upsz * V2 - 2u * Wm1),
                  (int)((sp - 3u) * (x.A3 - x.w3) + RB0 + upsz * V3 - 3u * Wm1));
   o2 = make_int4((int)x.W, (int)V2, (int)V3, 0);
+  if (p >= sz - 3) o1.x = o1.w = kTermNever;
+  if (p >= sz - 2) o0.w = o1.z = kTermNever;
+  if (p >= sz - 1) o0.x = o0.y = o0.z = o1.y = kTermNever;
 }
 #endif
 

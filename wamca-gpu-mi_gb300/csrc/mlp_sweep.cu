@@ -316,15 +316,22 @@ __global__ void __launch_bounds__(TL, CAP ? 1024 / TL : 1) k_sweep_dvnd(const Sw
 // Column terms are stored by the parity of their index so that the lanes of
 // a warp read consecutive 48-byte words (no bank conflicts).  Results are
 // identical to k_sweep_dvnd's.
+//
+// Bound by the L1 pipe (70 % of its wavefronts: the gather of D at scattered
+// columns and the column terms' reads) with 16 warps an SM (118 registers);
+// caps of 112 registers and fewer spill and lose 20 %.  What a row costs beyond
+// its deltas is therefore kept off the common case: minima are tracked only in
+// rows where some lane improves, the gather's columns are held in registers (no
+// index division, no client reads from shared memory), rows that have no pair
+// left are neither gathered nor evaluated.  1,024 searches of 100..1000 nodes
+// 107.4 -> 95.3 ms, 24 of them 11.0 -> 9.6 (both with their merges).
 template <int TLD, int TR>
 __global__ void __launch_bounds__(TLD / 2) k_sweep_dvnd2(const SweepTile* __restrict__ tiles,
                                                          const JobDev* __restrict__ jobs) {
   constexpr int NTH = TLD / 2;
-  constexpr int SR = TR + 3, SCV = TLD + 3, SC = TLD + 4, NT = TR + TLD + 5, NCS = TLD + TR - 1;
+  constexpr int SR = TR + 3, SC = TLD + 4, NT = TR + TLD + 5, NCS = TLD + TR - 1;
   constexpr int NCE = (NCS + 1) / 2;
   __shared__ __align__(16) int32_t sS[SR][SC];
-  __shared__ int32_t sRowT[SR];
-  __shared__ int32_t sColT[NT];
   __shared__ int4 sRt[TR][3];
   __shared__ int4 sCt[2][NCE][3];  // column term q at [q & 1][q >> 1]
 
@@ -342,21 +349,29 @@ __global__ void __launch_bounds__(TLD / 2) k_sweep_dvnd2(const SweepTile* __rest
   pdl_wait();
   pdl_launch_dependents();
   const bool done = stats[kStatConverged] || stats[kStatSweeps] >= stats[kStatLimit];
+  // Rows with a pair whose second position is at most sz - 2.
+  const int rows = min(TR, sz - 1 - L0 - r0);
+  const int lane = tid & 31;
+  constexpr int kM = (NT + NTH - 1) / NTH, kRow = (SR + 31) / 32, kX = (3 * SR + NTH - 1) / NTH;
+  int32_t col[kM], row[kRow], ext[kX];
+#pragma unroll
+  for (int m = 0; m < kM; m++) {
+    const int q = tid + m * NTH, p = r0 + L0 - 2 + q;
+    col[m] = (q < NT && p <= sz - 1) ? t[p] : -1;
+  }
+#pragma unroll
+  for (int u = 0; u < kRow; u++) {
+    const int q = lane + 32 * u, p = r0 - 1 + q;
+    row[u] = (q < SR && p <= sz - 1) ? t[p] * n : 0;
+  }
+#pragma unroll
+  for (int u = 0; u < kX; u++) {
+    const int e = tid + u * NTH, a = e / 3, rp = r0 - 1 + a, cp = rp + L0 - 1 + TLD + (e - 3 * a);
+    ext[u] = (a < SR && cp <= sz - 1) ? t[rp] * n + t[cp] : -1;
+  }
   {
-    constexpr int kSR = (SR + NTH - 1) / NTH, kNT = (NT + NTH - 1) / NTH;
     constexpr int kR = (3 * TR + NTH - 1) / NTH, kC = (3 * NCS + NTH - 1) / NTH;
-    int32_t vRT[kSR], vCT[kNT];
     int4 vR[kR], vC[kC];
-#pragma unroll
-    for (int u = 0; u < kSR; u++) {
-      const int q = tid + u * NTH, p = r0 - 1 + q;
-      vRT[u] = (q < SR && p <= sz - 1) ? t[p] : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < kNT; u++) {
-      const int q = tid + u * NTH, p = r0 + L0 - 2 + q;
-      vCT[u] = (q < NT && p <= sz - 1) ? t[p] : 0;
-    }
 #pragma unroll
     for (int u = 0; u < kR; u++) {
       const int q = tid + u * NTH, p = r0 + q / 3;
@@ -365,17 +380,8 @@ __global__ void __launch_bounds__(TLD / 2) k_sweep_dvnd2(const SweepTile* __rest
 #pragma unroll
     for (int u = 0; u < kC; u++) {
       const int q = tid + u * NTH, p = r0 + L0 + q / 3;
-      vC[u] = (q < 3 * NCS && p <= sz - 1) ? __ldg(CT + (size_t)p * 3 + q % 3) : make_int4(0, 0, 0, 0);
-    }
-#pragma unroll
-    for (int u = 0; u < kSR; u++) {
-      const int q = tid + u * NTH;
-      if (q < SR) sRowT[q] = vRT[u];
-    }
-#pragma unroll
-    for (int u = 0; u < kNT; u++) {
-      const int q = tid + u * NTH;
-      if (q < NT) sColT[q] = vCT[u];
+      const int never = q % 3 < 2 ? kTermNever : 0;
+      vC[u] = (q < 3 * NCS && p <= sz - 1) ? __ldg(CT + (size_t)p * 3 + q % 3) : make_int4(never, never, never, never);
     }
 #pragma unroll
     for (int u = 0; u < kR; u++) {
@@ -386,44 +392,48 @@ __global__ void __launch_bounds__(TLD / 2) k_sweep_dvnd2(const SweepTile* __rest
     for (int u = 0; u < kC; u++) {
       const int q = tid + u * NTH;
       if (q < 3 * NCS) {
-        const int col = q / 3;
-        sCt[col & 1][col >> 1][q % 3] = vC[u];
+        const int c = q / 3;
+        sCt[c & 1][c >> 1][q % 3] = vC[u];
       }
     }
   }
-  __syncthreads();
   if (done) return;
-  {
-    constexpr int NG = (SR * SCV + NTH - 1) / NTH, GB = 21;
+  // The tile's distances, rows 0 .. rows + 2.  Row a needs columns a .. a + TLD + 2
+  // of the tile's NT: a thread loads those congruent to its index (whose
+  // clients it holds), the last three of every row are loaded apart.
+  constexpr int GR = 6, KF = TLD / NTH;
 #pragma unroll
-    for (int u0 = 0; u0 < NG; u0 += GB) {
-      int32_t gv[GB];
+  for (int a0 = 0; a0 < SR; a0 += GR) {
+    if (a0 > rows + 2) break;
+    int32_t gv[GR][KF];
 #pragma unroll
-      for (int u = 0; u < GB; u++) {
-        const int idx = tid + (u0 + u) * NTH;
-        int32_t v = 0;
-        if (u0 + u < NG && idx < SR * SCV) {
-          const int a = idx / SCV, bb = idx - a * SCV;
-          const int rp = r0 - 1 + a, cp = rp + L0 - 1 + bb;
-          if (rp <= sz - 1 && cp <= sz - 1) v = __ldg(D + (size_t)sRowT[a] * n + sColT[a + bb]);
-        }
-        gv[u] = v;
-      }
+    for (int g = 0; g < GR; g++) {
+      const int a = a0 + g;
+      if (a >= SR) continue;
+      const int32_t ro = __shfl_sync(kFull, row[a >> 5], a & 31);
 #pragma unroll
-      for (int u = 0; u < GB; u++) {
-        const int idx = tid + (u0 + u) * NTH;
-        if (u0 + u < NG && idx < SR * SCV) {
-          const int a = idx / SCV, bb = idx - a * SCV;
-          sS[a][bb] = gv[u];
-        }
+      for (int f = 0; f < KF; f++) {
+        const int32_t c = tid >= a ? col[f] : tid + NTH >= a ? col[f + 1] : col[f + 2 < kM ? f + 2 : kM - 1];
+        gv[g][f] = c >= 0 ? __ldg(D + ro + c) : 0;
       }
     }
+#pragma unroll
+    for (int g = 0; g < GR; g++) {
+      const int a = a0 + g;
+      if (a >= SR) continue;
+      const int b0 = tid - a + (tid >= a ? 0 : tid + NTH >= a ? NTH : 2 * NTH);
+#pragma unroll
+      for (int f = 0; f < KF; f++) sS[a][b0 + f * NTH] = gv[g][f];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kX; u++) {
+    const int e = tid + u * NTH, a = e / 3;
+    if (a < SR) sS[a][TLD + (e - 3 * a)] = ext[u] >= 0 ? __ldg(D + ext[u]) : 0;
   }
   __syncthreads();
 
-  const int L = L0 + 2 * tid, b = 2 * tid + 1, lane = tid & 31;
-  const bool L2 = L >= 2;  // diagonal L + 1 >= 2 always
-  const int rows = min(TR, sz - 2 - r0);
+  const int L = L0 + 2 * tid, b = 2 * tid + 1;
   // Distances carried into row a: row a-1 at b+1, b+2 (x1, x2); row a at
   // b-1 .. b+2 (y0..y3); row a+1 at b+1, b+2 (z2, z3).
   uint32_t x1 = (uint32_t)sS[0][b + 1], x2 = (uint32_t)sS[0][b + 2];
@@ -438,6 +448,9 @@ __global__ void __launch_bounds__(TLD / 2) k_sweep_dvnd2(const SweepTile* __rest
   int d2A = 0, d2B = 0, dF1 = 0, dF2 = 0, dF3 = 0, dB1 = 0, dB2 = 0, dB3 = 0;
   uint64_t* keys = J->keys;
   const int nbS = nb_blocks(0, sz);
+  // Diagonal 1 has no swap: its value is raised to the top.
+  const int32_t swap_floor = L >= 2 ? (int32_t)0x80000000 : kInf32;
+  bool any = false;
 #pragma unroll 2
   for (int a = 1; a <= rows; a++) {
     // New distances: row a at b+3, row a+1 at b-1 and b, row a+2 at b+1 and b+2.
@@ -449,12 +462,10 @@ __global__ void __launch_bounds__(TLD / 2) k_sweep_dvnd2(const SweepTile* __rest
     // Column term of diagonal L + 1 (index a + 2 tid).
     const int4 N0 = sCt[a & 1][(a >> 1) + tid][0], N1 = sCt[a & 1][(a >> 1) + tid][1],
                N2 = sCt[a & 1][(a >> 1) + tid][2];
-    const int isc = (int)sc;
-    const bool v1 = isc >= 2, v2 = isc >= 3, v3 = isc >= 4, v4 = isc >= 5;
     const uint32_t P1 = sr * x1, P4 = (sc - 1u) * y2, Q1 = sr * x2, Q4 = (sc - 2u) * y3;
     const uint32_t sd = sc - 1u;  // s_c of diagonal L + 1
     // Diagonal L: e1 = x1, e2 = z0, e3 = y0, e4 = y2, e5 = y1, e6 = z2, e7 = y3, e8 = u1.
-    const int32_t dS = (int32_t)((sr - 1u) * z0 + sc * y0 + P1 + P4 + (uint32_t)R0.x + (uint32_t)K0.x);
+    const int32_t dS = max((int32_t)((sr - 1u) * z0 + sc * y0 + P1 + P4 + (uint32_t)R0.x + (uint32_t)K0.x), swap_floor);
     const int32_t d2 = (int32_t)(sc * (uint32_t)R2.x + sr * (uint32_t)K2.x + P1 + P4 + (uint32_t)R0.y + (uint32_t)K0.y);
     const int32_t f1 = (int32_t)(sc * y1 + P4 + (uint32_t)R0.z + (uint32_t)K0.z);
     const int32_t f2 = (int32_t)((sc - 2u) * z2 + sc * (y2 + (uint32_t)R2.y) + (uint32_t)R0.w + (uint32_t)K0.w);
@@ -471,68 +482,75 @@ __global__ void __launch_bounds__(TLD / 2) k_sweep_dvnd2(const SweepTile* __rest
     const int32_t k1 = (int32_t)((sr - 1u) * y2 + Q1 + (uint32_t)R1.y + (uint32_t)N1.y);
     const int32_t k2 = (int32_t)((sr - 2u) * y3 + sr * (uint32_t)N2.y + Q1 + (uint32_t)R1.z + (uint32_t)N1.z);
     const int32_t k3 = (int32_t)((sr - 3u) * y4 + sr * (uint32_t)N2.z + Q1 + (uint32_t)R1.w + (uint32_t)N1.w);
-
-    // swap: the row's blocks take the minimum over the warp's 64 pairs; ties
-    // to the lowest ctx (block A: lowest c; block B: highest c).
-    {
-      const uint32_t u0 = (v1 && L2) ? ((uint32_t)dS ^ 0x80000000u) : 0xffffffffu;
-      const uint32_t u1s = v2 ? ((uint32_t)eS ^ 0x80000000u) : 0xffffffffu;
-      const uint32_t um = min(u0, u1s);
-      const uint32_t mn = __reduce_min_sync(kFull, um);
-      if (mn < 0x80000000u) {
-        const unsigned ties = __ballot_sync(kFull, um == mn);
-        const int r = r0 + a - 1, c = r + L;
-        const int blkA = r - 1, blkB = sz - 3 - r;
-        if (blkA < nbS && lane == __ffs(ties) - 1) {
-          const bool first = u0 == mn;
-          atomicMin((unsigned long long*)&keys[blkA],
-                    (unsigned long long)make_key((int64_t)(first ? dS : eS), (uint32_t)(c + (first ? 0 : 1) - 3),
-                                                 kCtxBits));
-        }
-        if (blkB >= 0 && blkB < nbS && lane == 31 - __clz(ties)) {
-          const bool second = u1s == mn;
-          atomicMin((unsigned long long*)&keys[blkB],
-                    (unsigned long long)make_key((int64_t)(second ? eS : dS),
-                                                 (uint32_t)(sz - 2 - (c + (second ? 1 : 0))), kCtxBits));
+    // The rest is for rows with an improving move in some lane (a row of 64
+    // pairs, over a search: 17 % of them at n = 1000, 43 % at n = 200).
+    const int32_t sign = (dS | d2 | f1) | (f2 | f3 | g1) | (g2 | g3 | eS) | (e2 | h1 | h2) | (h3 | k1 | k2) | k3;
+    if (__any_sync(kFull, sign < 0)) {
+      any = true;
+      const int isc = (int)sc;
+      const bool v1 = isc >= 2, v2 = isc >= 3, v3 = isc >= 4, v4 = isc >= 5;
+      // swap: the row's blocks take the minimum over the warp's 64 pairs; ties
+      // to the lowest ctx (block A: lowest c; block B: highest c).
+      {
+        const uint32_t u0 = v1 ? ((uint32_t)dS ^ 0x80000000u) : 0xffffffffu;
+        const uint32_t u1s = v2 ? ((uint32_t)eS ^ 0x80000000u) : 0xffffffffu;
+        const uint32_t um = min(u0, u1s);
+        const uint32_t mn = __reduce_min_sync(kFull, um);
+        if (mn < 0x80000000u) {
+          const unsigned ties = __ballot_sync(kFull, um == mn);
+          const int r = r0 + a - 1, c = r + L;
+          const int blkA = r - 1, blkB = sz - 3 - r;
+          if (blkA < nbS && lane == __ffs(ties) - 1) {
+            const bool first = u0 == mn;
+            atomicMin((unsigned long long*)&keys[blkA],
+                      (unsigned long long)make_key((int64_t)(first ? dS : eS), (uint32_t)(c + (first ? 0 : 1) - 3),
+                                                   kCtxBits));
+          }
+          if (blkB >= 0 && blkB < nbS && lane == 31 - __clz(ties)) {
+            const bool second = u1s == mn;
+            atomicMin((unsigned long long*)&keys[blkB],
+                      (unsigned long long)make_key((int64_t)(second ? eS : dS),
+                                                   (uint32_t)(sz - 2 - (c + (second ? 1 : 0))), kCtxBits));
+          }
         }
       }
-    }
-    {
-      const bool lt = v1 && d2 < b2, le = v1 && d2 <= b2;
-      a2A = lt ? a : a2A;
-      a2B = le ? a : a2B;
-      b2 = lt ? d2 : b2;
-      const bool mt = v2 && e2 < c2, me = v2 && e2 <= c2;
-      d2A = mt ? a : d2A;
-      d2B = me ? a : d2B;
-      c2 = mt ? e2 : c2;
-    }
+      {
+        const bool lt = v1 && d2 < b2, le = v1 && d2 <= b2;
+        a2A = lt ? a : a2A;
+        a2B = le ? a : a2B;
+        b2 = lt ? d2 : b2;
+        const bool mt = v2 && e2 < c2, me = v2 && e2 <= c2;
+        d2A = mt ? a : d2A;
+        d2B = me ? a : d2B;
+        c2 = mt ? e2 : c2;
+      }
 #define MLP_TRACK_LT(v, d, best, arg) \
-  {                                   \
-    const bool up = (v) && (d) < (best); \
-    best = up ? (d) : best;           \
-    arg = up ? a : arg;               \
-  }
+    {                                   \
+      const bool up = (v) && (d) < (best); \
+      best = up ? (d) : best;           \
+      arg = up ? a : arg;               \
+    }
 #define MLP_TRACK_LE(v, d, best, arg) \
-  {                                   \
-    const bool up = (v) && (d) <= (best); \
-    best = up ? (d) : best;           \
-    arg = up ? a : arg;               \
-  }
-    MLP_TRACK_LT(v1, f1, bF1, aF1)
-    MLP_TRACK_LT(v2, f2, bF2, aF2)
-    MLP_TRACK_LT(v3, f3, bF3, aF3)
-    MLP_TRACK_LE(v1, g1, bB1, aB1)
-    MLP_TRACK_LE(v2, g2, bB2, aB2)
-    MLP_TRACK_LE(v3, g3, bB3, aB3)
-    MLP_TRACK_LT(v2, h1, cF1, dF1)
-    MLP_TRACK_LT(v3, h2, cF2, dF2)
-    MLP_TRACK_LT(v4, h3, cF3, dF3)
-    MLP_TRACK_LE(v2, k1, cB1, dB1)
-    MLP_TRACK_LE(v3, k2, cB2, dB2)
-    MLP_TRACK_LE(v4, k3, cB3, dB3)
+    {                                   \
+      const bool up = (v) && (d) <= (best); \
+      best = up ? (d) : best;           \
+      arg = up ? a : arg;               \
+    }
+      MLP_TRACK_LT(v1, f1, bF1, aF1)
+      MLP_TRACK_LT(v2, f2, bF2, aF2)
+      MLP_TRACK_LT(v3, f3, bF3, aF3)
+      MLP_TRACK_LE(v1, g1, bB1, aB1)
+      MLP_TRACK_LE(v2, g2, bB2, aB2)
+      MLP_TRACK_LE(v3, g3, bB3, aB3)
+      MLP_TRACK_LT(v2, h1, cF1, dF1)
+      MLP_TRACK_LT(v3, h2, cF2, dF2)
+      MLP_TRACK_LT(v4, h3, cF3, dF3)
+      MLP_TRACK_LE(v2, k1, cB1, dB1)
+      MLP_TRACK_LE(v3, k2, cB2, dB2)
+      MLP_TRACK_LE(v4, k3, cB3, dB3)
 #undef MLP_TRACK_LT
 #undef MLP_TRACK_LE
+    }
     x1 = y2;
     x2 = y3;
     y0 = z0;
@@ -547,6 +565,7 @@ __global__ void __launch_bounds__(TLD / 2) k_sweep_dvnd2(const SweepTile* __rest
     sr -= 1u;
     sc -= 1u;
   }
+  if (!any) return;
   publish_diagonal(keys, sz, r0, L, b2, a2A, a2B, bF1, bF2, bF3, aF1, aF2, aF3, bB1, bB2, bB3, aB1, aB2, aB3);
   publish_diagonal(keys, sz, r0, L + 1, c2, d2A, d2B, cF1, cF2, cF3, dF1, dF2, dF3, cB1, cB2, cB3, dB1, dB2, dB3);
 }
