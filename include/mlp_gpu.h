@@ -123,9 +123,10 @@ MLP_API int mlp_solver_set_stream(mlp_solver_t s, void* cuda_stream);
 /* Sweep tile shape index (0..13: diagonals x rows = 32x4, 32x8, 32x16, 64x4, 64x8,
  * 64x16, 128x8, 128x16, 32x32, 64x32, then 64x8, 64x16, 64x32, 128x16 where the
  * DVND sweep gives each thread two adjacent diagonals).  Loop mode of mlp_solver_dvnd: iterations = 0
- * (the default) runs the whole loop on the device (a CUDA-graph while node
- * over 16 iterations at a time, no host round trips; always the mode of
- * mlp_solver_dvnd_async; a solver without a stream of its own checks on the
+ * (the default) runs the whole loop on the device without host round trips
+ * (one launch for tours of up to 384 nodes, else a CUDA-graph while node over
+ * 16 iterations at a time, or up to eight iterations' launches; always the
+ * mode of mlp_solver_dvnd_async; a solver without a stream of its own checks on the
  * host after every iteration); iterations >= 1 replays CUDA graphs of that
  * many iterations and checks convergence on the host in between. */
 MLP_API int mlp_solver_set_tile_shape(mlp_solver_t s, int32_t shape);
@@ -136,8 +137,8 @@ MLP_API int mlp_solver_set_unroll(mlp_solver_t s, int32_t iterations);
  * identical; the switch exists for measurement and testing. */
 MLP_API int mlp_solver_set_sweep_kernel(mlp_solver_t s, int32_t variant);
 /* Merge kernel of the solver's iterations (as mlp_batch_set_merge_mode; the
- * default for one search is the six-CTA cluster).  Every mode gives the same
- * results. */
+ * default for one search is one CTA up to about 2,038 nodes, then the six-CTA
+ * cluster).  Every mode gives the same results. */
 MLP_API int mlp_solver_set_merge_mode(mlp_solver_t s, int32_t mode);
 /* Candidate mode of every later pass / DVND of this solver.  0 (default): one
  * candidate per reference block (the ODC kernels).  1: TOTAL multi-improvement
@@ -291,8 +292,8 @@ MLP_API int mlp_batch_reset(mlp_batch_t b);
 MLP_API int mlp_batch_result(mlp_batch_t b, int32_t job, int32_t* tour, int32_t len,
                              mlp_dvnd_stats_t* stats);
 MLP_API int mlp_batch_set_tile_shape(mlp_batch_t b, int32_t shape);
-/* Merge kernel of the batch's iterations: 0 = automatic (one CTA per job for
- * 16 jobs or more, otherwise a six-CTA cluster per job), 1 = cluster, 2 = one
+/* Merge kernel of the batch's iterations: 0 = automatic (one CTA per job up
+ * to 1,045 nodes and for 16 jobs or more, otherwise a six-CTA cluster per job), 1 = cluster, 2 = one
  * CTA per job.  Every mode gives the same results. */
 MLP_API int mlp_batch_set_merge_mode(mlp_batch_t b, int32_t mode);
 /* DVND sweep kernel of the batch's iterations (as mlp_solver_set_sweep_kernel). */

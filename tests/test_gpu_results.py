@@ -51,3 +51,37 @@ def test_batch_results_in_any_order(mlpgpu_mod):
     for q in (2, 0, 4, 3, 1, 2):
         t, st = b.result(q)
         assert np.array_equal(t, want[q][0]) and st["cost"] == want[q][1]["cost"]
+
+
+@pytest.mark.parametrize("n", [52, 420])
+@pytest.mark.parametrize("wide", [False, True])
+def test_under_stream_capture(mlpgpu_mod, n, wide):
+    """A capturing stream takes the reset and the sweep, and refuses a search, a
+    pass and a change of the mask, after which the solver works as before."""
+    torch = pytest.importorskip("torch")
+    x, y = oracle.uniform_instance(n, n)
+    t = oracle.random_perm_tour(n, n)
+    s = mlpgpu_mod.Solver(mlpgpu_mod.Problem.from_coords(x, y), wide=wide)
+    s.set_tour(t)
+    stream = torch.cuda.Stream()
+    assert mlpgpu_mod.lib().mlp_solver_set_stream(s._h, stream.cuda_stream) == 0
+    calls = [(lambda: s.begin(31, 5), True), (lambda: s.sweep(31, 1), True), (lambda: s.dvnd_async(31, 20), False),
+             (lambda: s.dvnd_async(31, 2), False), (lambda: s.pass_(1), False), (lambda: s.begin(1, 5), False)]
+    for call, taken in calls:
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                if taken:
+                    call()
+                else:
+                    with pytest.raises(Exception):
+                        call()
+            finally:
+                graph.capture_end()
+        s.set_tour(t)
+        want_tour, _ = oracle.dvnd(t, oracle.dist(x, y, True), wide)
+        s.dvnd()
+        assert np.array_equal(s.tour(), want_tour)
+        s.set_tour(t)

@@ -636,7 +636,14 @@ int JobSet::init() {
            "copy jobs");
   MLP_CUDA(cudaStreamSynchronize(stream_), "copy jobs");
   if (shape_ < 0) shape_ = default_shape(max_size_, (int)jobs_.size());
-  return small_search() ? kOk : ensure_tiles(dvnd_list());  // a one-launch search has no list
+  return ensure_lists();
+}
+
+// Both lists that a later call may launch from are built where shape and mask
+// are set, so that no launch has to (under stream capture it could not).
+int JobSet::ensure_lists() {
+  const int st = ensure_tiles(0);
+  return st != kOk || dvnd_list() == 0 ? st : ensure_tiles(dvnd_list());
 }
 
 int JobSet::ensure_tiles(int list, int buf, bool sync) {
@@ -729,7 +736,7 @@ int JobSet::set_shape(int shape) {
   shape_ = shape;
   drop_tiles();
   drop_graphs();
-  return djobs_ ? ensure_tiles(dvnd_list()) : kOk;
+  return djobs_ ? ensure_lists() : kOk;
 }
 
 int JobSet::set_unroll(int u) {
@@ -763,7 +770,7 @@ int JobSet::set_mask(int mask) {
   // these fields took a third of a neighbourhood pass (n = 100: 142 us, now 50
   // with its results read by one kernel; n = 1000: 190, now 62).
   MLP_CUDA(launch_set_fields(djobs_, (int)jobs_.size(), mask, 0, 0, stream_), "set mask");
-  return kOk;
+  return ensure_lists();
 }
 
 // Host state that follows the device's must not be changed by a call that is
@@ -827,7 +834,7 @@ int JobSet::set_total(bool on) {
   total_ = on;
   drop_tiles();
   drop_graphs();
-  return ensure_tiles(dvnd_list());
+  return ensure_lists();
 }
 
 int JobSet::launch_iteration() {

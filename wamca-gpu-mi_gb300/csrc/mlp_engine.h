@@ -195,6 +195,7 @@ class JobSet {
     int n = 0;
     bool ok = false;
   };
+  int ensure_lists();
   int ensure_tiles(int list, int buf = 0, bool sync = true);
   int dvnd_list() const { return sweep64() && !total_ ? 1 : 0; }  // the list of an iteration's sweep
   void drop_tiles() { lists_[0].ok = lists_[1].ok = false; }
