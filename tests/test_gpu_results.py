@@ -25,6 +25,31 @@ def test_recorded_pass_by_capacity(mlpgpu_mod, n, seed, wide):
             assert np.array_equal(s.tour(), want_tour)
 
 
+@pytest.mark.parametrize("n", [7, 255, 257, 700])
+@pytest.mark.parametrize("wide", [False, True])
+def test_candidates_leave_clean_keys(mlpgpu_mod, n, wide):
+    """Evaluations in any order, each from reset keys; Or-opt-k passes by capacity."""
+    x, y = oracle.clustered_instance(n, n)
+    t, D = oracle.random_perm_tour(n, n), oracle.dist(x, y, True)
+    s = mlpgpu_mod.Solver(mlpgpu_mod.Problem.from_coords(x, y), wide=wide)
+    s.set_tour(t)
+    for nb in (4, 0, 1, 0, 3, 2, 4):
+        c, i, j = s.eval(nb)
+        wc, wi, wj, _ = oracle.eval_nb(nb, t, D, wide)
+        assert np.array_equal(c, wc) and np.array_equal(i, wi) and np.array_equal(j, wj)
+    want_cost, want = s.pass_oropt(2)
+    want_tour = s.tour()
+    for cap in (0, 1, 1 << 15):
+        s.set_tour(t)
+        s.eval_oropt(2)
+        cost, moves = s.pass_oropt(2, max_moves=cap)
+        assert cost == want_cost == oracle.cost(want_tour, D, wide) and moves == want[:cap]
+        assert np.array_equal(s.tour(), want_tour)
+    want_tour, want = oracle.dvnd(want_tour, D, wide)
+    s.dvnd()
+    assert np.array_equal(s.tour(), want_tour)
+
+
 @pytest.mark.parametrize("n", [5, 100, 420])
 @pytest.mark.parametrize("iters", [1, 7, 8, 9])
 def test_few_iterations(mlpgpu_mod, n, iters):

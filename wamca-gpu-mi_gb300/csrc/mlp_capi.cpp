@@ -445,12 +445,8 @@ MLP_API int mlp_solver_eval(mlp_solver_t s, int32_t nb, int64_t* cost, int32_t* 
   MLP_TRY(s->set->set_mask(1 << nb));
   MLP_TRY(s->set->prepare(false));
   MLP_TRY(s->set->sweep_only());
-  std::vector<uint64_t> keys(m);
-  MLP_CUDA(cudaMemcpyAsync(keys.data(), s->job->dev.keys + off, sizeof(uint64_t) * m, cudaMemcpyDeviceToHost,
-                           s->set->stream()),
-           "copy keys");
-  MLP_TRY(s->set->prepare(false));
-  MLP_CUDA(cudaStreamSynchronize(s->set->stream()), "sync");
+  const uint64_t* keys;
+  MLP_TRY(s->set->take_keys(off, m, &keys));
   const int64_t sentinel = s->wide ? INT64_MAX : (int64_t)kCostInfty32;
   for (int b = 0; b < m; b++) {
     if (keys[b] == kKeyNone) {
@@ -489,12 +485,8 @@ MLP_API int mlp_solver_eval_oropt(mlp_solver_t s, int32_t k, int64_t* cost, int3
   if (!cost || !oi || !oj) return arg_error("null argument");
   const int sz = s->prob->size, m = oropt_blocks(k, sz);
   MLP_TRY(oropt_eval_keys(s, k));
-  std::vector<uint64_t> keys(m);
-  MLP_CUDA(cudaMemcpyAsync(keys.data(), s->job->dev.keys, sizeof(uint64_t) * m, cudaMemcpyDeviceToHost,
-                           s->set->stream()),
-           "copy keys");
-  MLP_TRY(s->set->prepare(false));
-  MLP_CUDA(cudaStreamSynchronize(s->set->stream()), "sync");
+  const uint64_t* keys;
+  MLP_TRY(s->set->take_keys(0, m, &keys));
   const int64_t sentinel = s->wide ? INT64_MAX : (int64_t)kCostInfty32;
   for (int b = 0; b < m; b++) {
     if (keys[b] == kKeyNone) {
@@ -536,22 +528,21 @@ MLP_API int mlp_solver_pass_oropt(mlp_solver_t s, int32_t k, int32_t max_moves, 
                              s->set->stream()),
            "Or-opt-k pass kernel");
   MLP_TRY(s->set->prepare(false));  // w, prefix arrays and cost of the new tour; keys reset
-  int applied = 0;
-  MLP_CUDA(cudaMemcpyAsync(&applied, dcnt, sizeof(int), cudaMemcpyDeviceToHost, s->set->stream()), "copy count");
-  MLP_CUDA(cudaStreamSynchronize(s->set->stream()), "sync");
-  const int take = std::min(applied, std::max(0, (int)max_moves));
-  if (take > 0) {
-    std::vector<uint32_t> mv(take);
-    MLP_CUDA(cudaMemcpyAsync(mv.data(), dij, 4 * take, cudaMemcpyDeviceToHost, s->set->stream()), "copy moves");
-    MLP_CUDA(cudaMemcpyAsync(costs, dcost, 8 * take, cudaMemcpyDeviceToHost, s->set->stream()), "copy moves");
-    MLP_CUDA(cudaStreamSynchronize(s->set->stream()), "sync");
-    for (int q = 0; q < take; q++) {
-      is[q] = (int32_t)(mv[q] & 0x3fff);
-      js[q] = (int32_t)(mv[q] >> 14);
-    }
+  const int cap = std::min(std::max(0, (int)max_moves), m);
+  const int64_t *head, *mc;
+  const uint32_t* mv;
+  MLP_TRY(s->set->read_oropt(dcnt, dij, dcost, cap, &head, &mc, &mv));
+  const int applied = (int)head[2], take = std::min(applied, cap);
+  for (int q = 0; q < take; q++) {
+    is[q] = (int32_t)(mv[q] & 0x3fff);
+    js[q] = (int32_t)(mv[q] >> 14);
+    costs[q] = mc[q];
   }
   if (count) *count = applied;
-  if (new_cost) MLP_TRY(mlp_solver_cost(s, new_cost));
+  if (new_cost) {
+    MLP_TRY(s->set->check_error(head[1]));
+    *new_cost = head[0];
+  }
   return kOk;
 }
 

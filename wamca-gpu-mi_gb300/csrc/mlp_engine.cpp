@@ -1199,6 +1199,24 @@ int JobSet::read_result(int job, bool tour, const int64_t** stats, const int32_t
   return check_error(hresult_[kStatWords]);
 }
 
+int JobSet::take_keys(int off, int m, const uint64_t** keys) {
+  uint64_t* out = reinterpret_cast<uint64_t*>(hresult_);
+  MLP_CUDA(launch_take_keys(djobs_, all_jobs_[0]->size, off, m, out, stream_), "read keys");
+  MLP_CUDA(cudaStreamSynchronize(stream_), "read keys");
+  *keys = out;
+  return kOk;
+}
+
+int JobSet::read_oropt(const int* count, const uint32_t* dmoves, const int64_t* dcosts, int cap, const int64_t** head,
+                       const int64_t** costs, const uint32_t** moves) {
+  MLP_CUDA(launch_oropt_result(dstats_, count, dmoves, dcosts, cap, hresult_, stream_), "read moves");
+  MLP_CUDA(cudaStreamSynchronize(stream_), "read moves");
+  *head = hresult_;
+  *costs = hresult_ + 3;
+  *moves = reinterpret_cast<const uint32_t*>(hresult_ + 3 + cap);
+  return kOk;
+}
+
 int JobSet::read_pass(int cap, const int64_t** stats, const int64_t** costs, const uint32_t** moves) {
   const Job* j = all_jobs_[0];
   MLP_CUDA(launch_pass_result(dstats_, j->dev.moves_out, j->dev.moves_cost, cap, hresult_, stream_), "read moves");

@@ -154,6 +154,12 @@ class JobSet {
   // tour, or a recorded pass's first `cap` moves, in pinned memory that holds
   // until the next of these calls.
   int read_result(int job, bool tour, const int64_t** stats, const int32_t** out);
+  // The first job's candidate keys [off, off + m) (all are reset), and an Or-opt-k
+  // pass's results, likewise.
+  int take_keys(int off, int m, const uint64_t** keys);
+  int read_oropt(const int* count, const uint32_t* dmoves, const int64_t* dcosts, int cap, const int64_t** head,
+                 const int64_t** costs, const uint32_t** moves);
+  int check_error(int64_t err);  // a statistics error word
   int read_pass(int cap, const int64_t** stats, const int64_t** costs, const uint32_t** moves);
   // run() is one device-side loop, which needs no wait between its iterations.
   bool loops_on_device() const { return device_loop_ && stream_ != 0 && all_jobs_.size() == 1; }
@@ -199,7 +205,6 @@ class JobSet {
   int ensure_tiles(int list, int buf = 0, bool sync = true);
   int dvnd_list() const { return sweep64() && !total_ ? 1 : 0; }  // the list of an iteration's sweep
   void drop_tiles() { lists_[0].ok = lists_[1].ok = false; }
-  int check_error(int64_t err);
   int refuse_capture(const char* what);
   int check_stats(const int64_t* hst);  // the statistics' internal error words
   void drop_graphs();

@@ -77,6 +77,13 @@ cudaError_t launch_set_fields(JobDev* jobs, int njobs, int nb_mask, int flags_on
 constexpr int kResultHead = kStatWords + 2;  // words before the tour
 cudaError_t launch_result(const int64_t* stats, int njobs, int job, const int32_t* tour, int size, int64_t* out,
                           cudaStream_t s);
+// One job's candidate keys [off, off + m) into mapped pinned memory; all of the
+// job's keys are reset.
+cudaError_t launch_take_keys(const JobDev* job, int size, int off, int m, uint64_t* out, cudaStream_t s);
+// An Or-opt-k pass's cost and move count, then its first min(count, cap) moves:
+// cap 64-bit costs, cap 32-bit moves.
+cudaError_t launch_oropt_result(const int64_t* stats, const int* count, const uint32_t* moves, const int64_t* costs, int cap,
+                                int64_t* out, cudaStream_t s);
 // The same after a recorded pass: statistics, then the first min(moves, cap)
 // moves: cap 64-bit costs, cap 32-bit moves.
 cudaError_t launch_pass_result(const int64_t* stats, const uint32_t* moves, const int64_t* costs, int cap, int64_t* out,
