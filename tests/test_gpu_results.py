@@ -78,6 +78,21 @@ def test_batch_results_in_any_order(mlpgpu_mod):
         assert np.array_equal(t, want[q][0]) and st["cost"] == want[q][1]["cost"]
 
 
+def test_batch_results_from_threads(mlpgpu_mod):
+    from concurrent.futures import ThreadPoolExecutor
+
+    b = mlpgpu_mod.Batch()
+    for q in range(24):
+        x, y = oracle.uniform_instance(30 + 17 * q, q)
+        b.add(mlpgpu_mod.Problem.from_coords(x, y), oracle.random_perm_tour(30 + 17 * q, q))
+    b.run()
+    want = [b.result(q) for q in range(24)]
+    with ThreadPoolExecutor(8) as pool:
+        got = list(pool.map(lambda q: b.result(q % 24), range(960)))
+    for q, (t, st) in enumerate(got):
+        assert np.array_equal(t, want[q % 24][0]) and st == want[q % 24][1]
+
+
 @pytest.mark.parametrize("n", [52, 420])
 @pytest.mark.parametrize("wide", [False, True])
 def test_under_stream_capture(mlpgpu_mod, n, wide):

@@ -899,6 +899,7 @@ MLP_API int mlp_batch_result(mlp_batch_t b, int32_t job, int32_t* tour, int32_t 
   }
   const int64_t* st;
   const int32_t* t;
+  std::lock_guard<std::mutex> lock(b->set->result_mutex());
   const int status = b->set->read_result(job, tour != nullptr, &st, &t);
   if (status == kErrCuda) return status;
   if (tour) std::memcpy(tour, t, sizeof(int32_t) * j->size);

@@ -636,15 +636,13 @@ int JobSet::init() {
            "copy jobs");
   MLP_CUDA(cudaStreamSynchronize(stream_), "copy jobs");
   if (shape_ < 0) shape_ = default_shape(max_size_, (int)jobs_.size());
-  return ensure_lists();
+  return ensure_list();
 }
 
-// Both lists that a later call may launch from are built where shape and mask
-// are set, so that no launch has to (under stream capture it could not).
-int JobSet::ensure_lists() {
-  const int st = ensure_tiles(0);
-  return st != kOk || dvnd_list() == 0 ? st : ensure_tiles(dvnd_list());
-}
+// The list that the sweeps of the set's shape, mask and candidate mode launch
+// from is built where these are set, so that no launch has to (under stream
+// capture it could not).
+int JobSet::ensure_list() { return ensure_tiles(dvnd_list()); }
 
 int JobSet::ensure_tiles(int list, int buf, bool sync) {
   TileList& l = lists_[list];
@@ -736,7 +734,7 @@ int JobSet::set_shape(int shape) {
   shape_ = shape;
   drop_tiles();
   drop_graphs();
-  return djobs_ ? ensure_lists() : kOk;
+  return djobs_ ? ensure_list() : kOk;
 }
 
 int JobSet::set_unroll(int u) {
@@ -770,7 +768,7 @@ int JobSet::set_mask(int mask) {
   // these fields took a third of a neighbourhood pass (n = 100: 142 us, now 50
   // with its results read by one kernel; n = 1000: 190, now 62).
   MLP_CUDA(launch_set_fields(djobs_, (int)jobs_.size(), mask, 0, 0, stream_), "set mask");
-  return ensure_lists();
+  return ensure_list();
 }
 
 // Host state that follows the device's must not be changed by a call that is
@@ -834,7 +832,7 @@ int JobSet::set_total(bool on) {
   total_ = on;
   drop_tiles();
   drop_graphs();
-  return ensure_lists();
+  return ensure_list();
 }
 
 int JobSet::launch_iteration() {

@@ -16,6 +16,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -153,6 +154,9 @@ class JobSet {
   // Waits for the stream and returns one job's statistics and, on request, its
   // tour, or a recorded pass's first `cap` moves, in pinned memory that holds
   // until the next of these calls.
+  // Held from read_result until its output is copied: threads may read a set's
+  // results at the same time.
+  std::mutex& result_mutex() { return result_mu_; }
   int read_result(int job, bool tour, const int64_t** stats, const int32_t** out);
   // The first job's candidate keys [off, off + m) (all are reset), and an Or-opt-k
   // pass's results, likewise.
@@ -201,7 +205,7 @@ class JobSet {
     int n = 0;
     bool ok = false;
   };
-  int ensure_lists();
+  int ensure_list();
   int ensure_tiles(int list, int buf = 0, bool sync = true);
   int dvnd_list() const { return sweep64() && !total_ ? 1 : 0; }  // the list of an iteration's sweep
   void drop_tiles() { lists_[0].ok = lists_[1].ok = false; }
@@ -239,6 +243,7 @@ class JobSet {
   JobDev* djobs_ = nullptr;
   TileList lists_[2];
   int64_t* hstats_ = nullptr;  // pinned, kStatWords per job
+  std::mutex result_mu_;
   int64_t* hresult_ = nullptr;  // behind it: room for one job's results
   int64_t* hstats2_ = nullptr;  // a second one (the batch loop reads one while the other fills)
   cudaEvent_t stats_ev_[2] = {nullptr, nullptr};
