@@ -564,7 +564,10 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kMergeThr
   const JobDev* J = jobs + blockIdx.x / kClusterCtas;
   {
     const int64_t* stt = J->stats;
-    if (stt[kStatConverged] || stt[kStatSweeps] >= stt[kStatLimit]) return;  // the whole cluster
+    if (stt[kStatConverged] || stt[kStatSweeps] >= stt[kStatLimit]) {  // the whole cluster
+      pdl_wait();  // see launch_pdl
+      return;
+    }
   }
   const int sz = J->size, mask = J->nb_mask, tid = threadIdx.x, nt = blockDim.x;
   const MergeLayout lay(sz);
@@ -758,9 +761,9 @@ __global__ void __launch_bounds__(kSoloThreads) k_merge_solo(const JobDev* __res
   const JobDev* J = jobs + blockIdx.x;
   {
     const int64_t* stt = J->stats;
+    pdl_wait();  // the sweep's keys
     if (stt[kStatConverged] || stt[kStatSweeps] >= stt[kStatLimit]) return;
   }
-  pdl_wait();  // the sweep's keys
   const int sz = J->size, mask = J->nb_mask, tid = threadIdx.x, nt = blockDim.x;
   const SoloLayout lay(sz);
   uint8_t* ws = use_smem ? dsm : J->ws;
@@ -953,9 +956,9 @@ __global__ void __launch_bounds__(kMergeThreads) k_total_finish(const JobDev* __
   const JobDev* J = jobs + blockIdx.x;
   {
     const int64_t* stt = J->stats;
+    pdl_wait();  // the greedy's kept moves
     if (stt[kStatConverged] || stt[kStatSweeps] >= stt[kStatLimit]) return;
   }
-  pdl_wait();  // the greedy's kept moves
   const int sz = J->size, mask = J->nb_mask, tid = threadIdx.x, nt = blockDim.x;
   const SoloLayout lay(sz);
   uint8_t* ws = use_smem ? dsm : J->ws;

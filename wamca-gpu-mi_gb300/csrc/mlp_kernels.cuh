@@ -24,8 +24,11 @@ constexpr int kNumTileShapes = sizeof(kTileShapes) / sizeof(kTileShapes[0]);
 // stream (an ordinary launch on the legacy default stream): it may start
 // while its predecessor runs, once that predecessor calls
 // pdl_launch_dependents, and must call pdl_wait before it reads anything the
-// predecessor writes.  In a captured graph the dependency becomes a
-// programmatic edge.
+// predecessor writes.  Every thread also calls it before it returns, with or
+// without work: a kernel's end then implies its predecessors' ends, on which
+// its successors rely (of two merges of one sweep, the second may read the
+// sweep's keys although it waits for the first alone).  In a captured graph the
+// dependency becomes a programmatic edge.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg = {};

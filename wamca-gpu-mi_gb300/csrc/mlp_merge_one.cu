@@ -354,7 +354,10 @@ __global__ void __launch_bounds__(NT) k_merge_one(const JobDev* __restrict__ job
   const JobDev* Jg = jobs + blockIdx.x;
   {
     const int64_t* stt = Jg->stats;
-    if (stt[kStatConverged] || stt[kStatSweeps] >= stt[kStatLimit]) return;
+    if (stt[kStatConverged] || stt[kStatSweeps] >= stt[kStatLimit]) {
+      pdl_wait();  // see launch_pdl
+      return;
+    }
   }
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   constexpr int nt = NT;

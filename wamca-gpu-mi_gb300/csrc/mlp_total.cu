@@ -338,12 +338,16 @@ __global__ void __launch_bounds__(kTotThreads) k_total_select(const JobDev* __re
   // and neighbourhood).
   {
     const int64_t* stt = J->stats;
-    if (stt[kStatConverged] || stt[kStatSweeps] >= stt[kStatLimit]) return;
+    if (stt[kStatConverged] || stt[kStatSweeps] >= stt[kStatLimit]) {
+      pdl_wait();  // see launch_pdl
+      return;
+    }
   }
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
   const int sz = J->size;
   if (!((J->nb_mask >> nb) & 1)) {
     if (first && tid == 0) J->tkcount[nb] = 0;
+    pdl_wait();
     return;
   }
   pdl_wait();  // the collecting sweep's lists
