@@ -1,0 +1,64 @@
+// host_faults.cpp -- the engine's host code on a fake CUDA runtime: what a call
+// answers when a launch or an allocation fails, and what it does on a stream
+// that is being captured.  One check a run (argv[1]); exit status 0 = it holds.
+#include "fake_cuda.h"
+
+#include <vector>
+
+#include "mlp_gpu.h"
+
+#define REQUIRE(c)                                                                 \
+  do {                                                                             \
+    if (!(c)) {                                                                    \
+      std::fprintf(stderr, "%s:%d: %s (%s)\n", __FILE__, __LINE__, #c, mlp_last_error()); \
+      return 1;                                                                    \
+    }                                                                              \
+  } while (0)
+
+static mlp_problem_t problem(int n, int dmax) {
+  std::vector<int32_t> D((size_t)n * n);
+  for (int a = 0; a < n; a++)
+    for (int b = 0; b < n; b++) D[(size_t)a * n + b] = a == b ? 0 : 1 + (a * 7 + b * 7) % dmax;
+  D[1] = D[n] = dmax;
+  mlp_problem_t p = nullptr;
+  return mlp_problem_create_matrix(n, D.data(), 1, &p) == 0 ? p : nullptr;
+}
+
+static std::vector<int32_t> tour(int n) {
+  std::vector<int32_t> t(n + 1, 0);
+  for (int q = 0; q < n; q++) t[q] = q;
+  return t;
+}
+
+// A batch's result is not read when its kernel could not be launched.
+static int batch_result() {
+  const int n = 50;
+  mlp_batch_t b = nullptr;
+  mlp_problem_t p = problem(n, 100);
+  REQUIRE(p && mlp_batch_create(0, &b) == 0);
+  int32_t job = -1;
+  const std::vector<int32_t> t = tour(n);
+  REQUIRE(mlp_batch_add(b, p, t.data(), n + 1, &job) == 0 && mlp_batch_reset(b) == 0);
+  for (const char* what : {"launch_result", "cudaStreamSynchronize"})
+    for (const cudaError_t e : {cudaErrorMemoryAllocation, cudaErrorLaunchFailure}) {
+      fake::fail(what, e);
+      std::vector<int32_t> out(n + 1, -7);
+      mlp_dvnd_stats_t st;
+      const int want = e == cudaErrorMemoryAllocation ? MLP_ERR_NOMEM : MLP_ERR_CUDA;
+      REQUIRE(mlp_batch_result(b, job, out.data(), n + 1, nullptr) == want);
+      REQUIRE(mlp_batch_result(b, job, out.data(), n + 1, &st) == want);
+      for (int32_t v : out) REQUIRE(v == -7);
+      fake::fails.clear();
+      REQUIRE(mlp_batch_result(b, job, out.data(), n + 1, &st) == 0);
+    }
+  mlp_batch_destroy(b);
+  mlp_problem_destroy(p);
+  return 0;
+}
+
+int main(int argc, char** argv) {
+  const std::string check = argc > 1 ? argv[1] : "";
+  if (check == "batch_result") return batch_result();
+  std::fprintf(stderr, "unknown check\n");
+  return 2;
+}

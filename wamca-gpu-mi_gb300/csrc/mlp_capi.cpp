@@ -897,11 +897,13 @@ MLP_API int mlp_batch_result(mlp_batch_t b, int32_t job, int32_t* tour, int32_t 
   if (tour) {
     if (len < j->size) return arg_error("buffer shorter than size");
   }
-  const int64_t* st;
-  const int32_t* t;
+  const int64_t* st = nullptr;
+  const int32_t* t = nullptr;
   std::lock_guard<std::mutex> lock(b->set->result_mutex());
+  // With an error that a search reported the results are there, and a call for
+  // the tour alone takes it.
   const int status = b->set->read_result(job, tour != nullptr, &st, &t);
-  if (status == kErrCuda) return status;
+  if (st == nullptr) return status;
   if (tour) std::memcpy(tour, t, sizeof(int32_t) * j->size);
   if (stats) {
     MLP_TRY(status);

@@ -1189,6 +1189,8 @@ int JobSet::read_stats(std::vector<std::array<int64_t, kStatWords>>* out) {
 
 int JobSet::read_result(int job, bool tour, const int64_t** stats, const int32_t** out) {
   const Job* j = all_jobs_[job];
+  *stats = nullptr;
+  *out = nullptr;
   MLP_CUDA(launch_result(dstats_, (int)all_jobs_.size(), job, tour ? j->dev.tour : nullptr, j->size, hresult_, stream_),
            "read result");
   MLP_CUDA(cudaStreamSynchronize(stream_), "read result");

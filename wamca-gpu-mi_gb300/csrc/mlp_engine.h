@@ -151,12 +151,13 @@ class JobSet {
   // synchronisation.  Read the results with read_stats().
   int enqueue_device_loop(int max_iters);
   int read_stats(std::vector<std::array<int64_t, kStatWords>>* out);
-  // Waits for the stream and returns one job's statistics and, on request, its
-  // tour, or a recorded pass's first `cap` moves, in pinned memory that holds
-  // until the next of these calls.
   // Held from read_result until its output is copied: threads may read a set's
   // results at the same time.
   std::mutex& result_mutex() { return result_mu_; }
+  // Waits for the stream and returns one job's statistics and, on request, its
+  // tour, or a recorded pass's first `cap` moves, in pinned memory that holds
+  // until the next of these calls (read_result: null pointers where nothing
+  // could be read).
   int read_result(int job, bool tour, const int64_t** stats, const int32_t** out);
   // The first job's candidate keys [off, off + m) (all are reset), and an Or-opt-k
   // pass's results, likewise.
