@@ -56,9 +56,55 @@ static int batch_result() {
   return 0;
 }
 
+// The sweeps of a solver launch on a capturing stream whatever was switched
+// before or during the capture: no tile list is left to be built by a launch.
+static int captured_sweeps() {
+  const int n = 400;
+  mlp_problem_t p = problem(n, 65535);  // 64-bit costs that leave 32 bits
+  for (int wide = 0; wide < 2; wide++)
+    for (int shape = -1; shape < 14; shape++) {
+      mlp_solver_t s = nullptr;
+      REQUIRE(p && mlp_solver_create(p, wide, &s) == 0);
+      const std::vector<int32_t> t = tour(n);
+      REQUIRE(mlp_solver_set_tour(s, t.data(), n + 1) == 0);
+      if (shape >= 0) REQUIRE(mlp_solver_set_tile_shape(s, shape) == 0);
+      auto sweep = [&] {
+        fake::capturing = true;
+        const int st = mlp_solver_sweep(s, MLP_NB_ALL, 1, nullptr);
+        fake::capturing = false;
+        return st;
+      };
+      REQUIRE(sweep() == 0);
+      for (int variant : {0, 1, 0}) {
+        REQUIRE(mlp_solver_set_sweep_kernel(s, variant) == 0);
+        REQUIRE(sweep() == 0);
+      }
+      for (int variant : {1, 0, 1}) {
+        fake::capturing = true;
+        const int st = mlp_solver_set_sweep_kernel(s, variant);
+        fake::capturing = false;
+        REQUIRE(st == 0 && sweep() == 0);
+      }
+      for (int on : {1, 0}) {
+        REQUIRE(mlp_solver_set_total(s, on) == 0);
+        for (int variant : {0, 1}) {
+          REQUIRE(mlp_solver_set_sweep_kernel(s, variant) == 0);
+          REQUIRE(sweep() == 0);
+        }
+      }
+      // A mask set outside the capture.
+      REQUIRE(mlp_solver_sweep(s, 1, 1, nullptr) == 0 && mlp_solver_sweep(s, MLP_NB_ALL, 1, nullptr) == 0);
+      REQUIRE(sweep() == 0);
+      mlp_solver_destroy(s);
+    }
+  mlp_problem_destroy(p);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string check = argc > 1 ? argv[1] : "";
   if (check == "batch_result") return batch_result();
+  if (check == "captured_sweeps") return captured_sweeps();
   std::fprintf(stderr, "unknown check\n");
   return 2;
 }

@@ -30,3 +30,7 @@ def _run(exe, check):
 
 def test_failed_batch_result(exe):
     _run(exe, "batch_result")
+
+
+def test_sweeps_on_a_capturing_stream(exe):
+    _run(exe, "captured_sweeps")

@@ -639,10 +639,14 @@ int JobSet::init() {
   return ensure_list();
 }
 
-// The list that the sweeps of the set's shape, mask and candidate mode launch
-// from is built where these are set, so that no launch has to (under stream
-// capture it could not).
-int JobSet::ensure_list() { return ensure_tiles(dvnd_list()); }
+// The lists that the set's sweeps can launch from are built with the set and
+// where its shape changes, so that no launch has to, whatever mask, sweep kernel
+// or candidate mode it comes with (under stream capture it could not).  Only a
+// set whose active jobs changed builds the others when they are needed.
+int JobSet::ensure_list() {
+  const int st = ensure_tiles(0);
+  return st != kOk || !may_sweep64() ? st : ensure_tiles(wide_list());
+}
 
 int JobSet::ensure_tiles(int list, int buf, bool sync) {
   TileList& l = lists_[list];
@@ -903,12 +907,12 @@ int JobSet::sweep_only() {
 }
 
 int JobSet::sweep_kernel() {
-  const int st = ensure_tiles(sweep64() ? 1 : 0);
+  const int st = ensure_tiles(sweep64() ? wide_list() : 0);
   return st != kOk ? st : launch_dvnd_sweep();
 }
 
 int JobSet::launch_dvnd_sweep() {
-  const TileList& l = lists_[sweep64() ? 1 : 0];
+  const TileList& l = lists_[sweep64() ? wide_list() : 0];
   if (sweep64())
     MLP_CUDA(launch_sweep_dvnd_wide(l.d, l.n, djobs_, wide_shape(shape_), stream_), "sweep kernel");
   else if (dvnd_sweep())
@@ -985,7 +989,7 @@ static bool fits32(const Job* j) { return (int64_t)j->prob->dmax * j->size * j->
 // deltas modulo 2^32 are then the exact ones (n = 1000: 27.3 -> 22.5 us an
 // iteration).  A 64-bit batch has no 32-bit term tables: its sweep is the
 // 64-bit one.
-bool JobSet::sweep32() const { return !wide_ || (local_terms() && fits32(all_jobs_[0])); }
+bool JobSet::may_sweep64() const { return wide_ && !(local_terms() && fits32(all_jobs_[0])); }
 
 // The one-launch search applies: one search over all neighbourhoods, with the
 // default merge and sweep, whose distances fit a CTA's shared memory.

@@ -197,8 +197,7 @@ class JobSet {
 
  private:
   // The tile list of a sweep: list 0 in the set's shape, list 1 in the shape
-  // of the 64-bit DVND sweep.  Built when first needed; set_active and
-  // set_shape invalidate them.
+  // of the 64-bit DVND sweep where that is another one.
   struct TileList {
     SweepTile* d = nullptr;
     SweepTile* h[2] = {nullptr, nullptr};  // pinned staging
@@ -208,7 +207,8 @@ class JobSet {
   };
   int ensure_list();
   int ensure_tiles(int list, int buf = 0, bool sync = true);
-  int dvnd_list() const { return sweep64() && !total_ ? 1 : 0; }  // the list of an iteration's sweep
+  int wide_list() const { return wide_shape(shape_) == shape_ ? 0 : 1; }  // the list of the 64-bit DVND sweep
+  int dvnd_list() const { return sweep64() && !total_ ? wide_list() : 0; }  // the list of an iteration's sweep
   void drop_tiles() { lists_[0].ok = lists_[1].ok = false; }
   int refuse_capture(const char* what);
   int check_stats(const int64_t* hst);  // the statistics' internal error words
@@ -217,8 +217,8 @@ class JobSet {
   // in 32 bits (32-bit jobs, and one 64-bit search whose costs fit 32 bits) or
   // in 64.
   bool dvnd_sweep() const { return sweep_variant_ == 1 && mask_ == 0x1f; }
-  bool sweep32() const;
-  bool sweep64() const { return dvnd_sweep() && !sweep32(); }
+  bool may_sweep64() const;
+  bool sweep64() const { return dvnd_sweep() && may_sweep64(); }
   // A set of one search computes the DVND sweep's row and column terms in
   // every tile instead of having the ADS rebuild (one CTA, on the merge's
   // critical path) write term tables.
