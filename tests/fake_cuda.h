@@ -18,14 +18,18 @@
 namespace fake {
 std::map<std::string, int> calls;                  // calls by name
 std::map<std::string, std::pair<int, int>> fails;  // name -> (calls that still succeed, error)
+bool once = false;                                 // an armed failure happens once
+int held = 0;                                      // stream-ordered allocations not freed
 bool capturing = false;
 const void* grasp_table = nullptr;                 // the last launch_grasp's table
 
 inline cudaError_t call(const char* name) {
   calls[name]++;
   const auto f = fails.find(name);
-  if (f != fails.end() && f->second.first-- <= 0) return (cudaError_t)f->second.second;
-  return cudaSuccess;
+  if (f == fails.end() || f->second.first-- > 0) return cudaSuccess;
+  const cudaError_t e = (cudaError_t)f->second.second;
+  if (once) fails.erase(f);
+  return e;
 }
 inline void fail(const char* name, cudaError_t e, int after = 0) { fails[name] = {after, (int)e}; }
 inline cudaError_t no_capture(const char* name) { return capturing ? cudaErrorStreamCaptureUnsupported : call(name); }
@@ -44,7 +48,7 @@ cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1;
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return fake::call(__func__); }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return fake::no_capture(__func__); }
 cudaError_t cudaFree(void* p) { std::free(p); return fake::no_capture(__func__); }
-cudaError_t cudaFreeAsync(void* p, cudaStream_t) { std::free(p); return fake::call(__func__); }
+cudaError_t cudaFreeAsync(void* p, cudaStream_t) { std::free(p); fake::held -= p != nullptr; return fake::call(__func__); }
 cudaError_t cudaFreeHost(void* p) { std::free(p); return fake::no_capture(__func__); }
 cudaError_t cudaGetDevice(int* d) { *d = 0; return fake::call(__func__); }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 152; return fake::call(__func__); }
@@ -64,7 +68,11 @@ cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return fake::call(_
 cudaError_t cudaHostAlloc(void** p, size_t b, unsigned) { return fake::alloc(__func__, p, b); }
 cudaError_t cudaMallocHost(void** p, size_t b) { return fake::alloc(__func__, p, b); }
 cudaError_t cudaMalloc(void** p, size_t b) { return fake::alloc(__func__, p, b); }
-cudaError_t cudaMallocAsync(void** p, size_t b, cudaStream_t) { return fake::alloc(__func__, p, b); }
+cudaError_t cudaMallocAsync(void** p, size_t b, cudaStream_t) {
+  const cudaError_t e = fake::alloc(__func__, p, b);
+  fake::held += e == cudaSuccess;
+  return e;
+}
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t b, cudaMemPool_t, cudaStream_t) { return fake::alloc(__func__, p, b); }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t b, cudaMemcpyKind) { std::memcpy(d, s, b); return fake::no_capture(__func__); }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t b, cudaMemcpyKind, cudaStream_t) { std::memcpy(d, s, b); return fake::call(__func__); }

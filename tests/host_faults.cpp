@@ -101,10 +101,44 @@ static int captured_sweeps() {
   return 0;
 }
 
+// Starts are built whichever allocation of the ordered rows fails; any other
+// failing allocation is reported.
+static int constructor_memory() {
+  const int n = 50;
+  mlp_problem_t p = problem(n, 100);
+  REQUIRE(p != nullptr);
+  const uint32_t seed = 3;
+  std::vector<int32_t> t(n + 1);
+  fake::calls.clear();
+  REQUIRE(mlp_problem_random_tours(p, 1, &seed, 0.5f, t.data()) == 0 && fake::grasp_table != nullptr);
+  const int allocs = fake::calls["cudaMallocAsync"], sorts = fake::calls["launch_grasp_sort"];
+  REQUIRE(allocs == 5 && sorts == 1);  // tours, tasks, flag; the rows' jobs and table
+  for (int k = 0; k < allocs; k++)
+    for (bool all : {false, true}) {  // the k-th alone fails, or all from it on
+      fake::calls.clear();
+      fake::fail("cudaMallocAsync", cudaErrorMemoryAllocation, k);
+      fake::once = !all;
+      fake::grasp_table = &fake::calls;
+      const int st = mlp_problem_random_tours(p, 1, &seed, 0.5f, t.data());
+      fake::fails.clear();
+      fake::once = false;
+      if (k < 3) {
+        REQUIRE(st == MLP_ERR_NOMEM && fake::calls["launch_grasp"] == 0);
+      } else {
+        REQUIRE(st == 0 && fake::grasp_table == nullptr);
+        REQUIRE(fake::calls["launch_grasp"] == 1 && fake::calls["launch_grasp_sort"] == 0);
+      }
+      REQUIRE(fake::held == 0);
+    }
+  mlp_problem_destroy(p);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string check = argc > 1 ? argv[1] : "";
   if (check == "batch_result") return batch_result();
   if (check == "captured_sweeps") return captured_sweeps();
+  if (check == "constructor_memory") return constructor_memory();
   std::fprintf(stderr, "unknown check\n");
   return 2;
 }

@@ -34,3 +34,7 @@ def test_failed_batch_result(exe):
 
 def test_sweeps_on_a_capturing_stream(exe):
     _run(exe, "captured_sweeps")
+
+
+def test_constructor_memory(exe):
+    _run(exe, "constructor_memory")

@@ -539,12 +539,15 @@ int build_random_tours(const std::vector<GraspTask>& tasks, cudaStream_t stream)
            "copy constructor tasks");
   MLP_CUDA(cudaMemsetAsync(b.err, 0, sizeof(int), stream), "memset(constructor flag)");
   if (ncanon > 0) {
-    // Without room for the ordered rows the starts select from unsorted ones.
-    if (cudaMallocAsync(&b.table, sizeof(uint16_t) * (size_t)entries, stream) != cudaSuccess) {
+    // Without room for the ordered rows, or for their sort's jobs, the starts
+    // select from unsorted ones.
+    if (cudaMallocAsync(&b.sorts, sizeof(GraspSortJob) * sorts.size(), stream) != cudaSuccess) {
+      cudaGetLastError();
+      b.sorts = nullptr;
+    } else if (cudaMallocAsync(&b.table, sizeof(uint16_t) * (size_t)entries, stream) != cudaSuccess) {
       cudaGetLastError();
       b.table = nullptr;
     } else {
-      MLP_CUDA(cudaMallocAsync(&b.sorts, sizeof(GraspSortJob) * sorts.size(), stream), "cudaMallocAsync(constructor rows)");
       MLP_CUDA(cudaMemcpyAsync(b.sorts, sorts.data(), sizeof(GraspSortJob) * sorts.size(), cudaMemcpyHostToDevice, stream),
                "copy constructor rows");
       MLP_CUDA(launch_grasp_sort(b.sorts, (int)sorts.size(), nrows, max_n, b.table, stream), "constructor rows kernel");
