@@ -111,6 +111,12 @@ MLP_API int mlp_problem_random_tours(mlp_problem_t p, int32_t count, const uint3
  * std::sort (one warp per start, the sort on one lane; slower, for parity). */
 MLP_API int mlp_problem_random_tours_ties(mlp_problem_t p, int32_t count, const uint32_t* seeds, float alpha,
                                           int32_t ties, int32_t* tours);
+/* How later starts of this problem with ties = 0 are built (no counterpart in
+ * the reference): 0 (default) automatic, 1 from rows ordered once per call (2
+ * n^2 bytes of scratch during it; without room for them as 2), 2 by selection
+ * from unsorted rows.  Results are identical; the switch exists for measurement
+ * and testing. */
+MLP_API int mlp_problem_set_start_rows(mlp_problem_t p, int32_t mode);
 /* Copies the n x n distance matrix to host memory. */
 MLP_API int mlp_problem_get_dist(mlp_problem_t p, int32_t* dist);
 MLP_API void mlp_problem_destroy(mlp_problem_t p);

@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,shape", [(60, 0), (420, -1), (420, 5)])
-def test_sweep_kernels_under_capture(mlpgpu_mod, n, shape):
+@pytest.mark.parametrize("before,inside", [((), None), ((0,), None), ((), 0), ((0,), 1), ((0, 1), None)])
+@pytest.mark.parametrize("total", [False, True])
+def test_sweep_kernels_under_capture(mlpgpu_mod, n, shape, before, inside, total):
     torch = pytest.importorskip("torch")
     r = np.random.default_rng(n)
     D = np.triu(r.integers(0, 65536, (n, n)), 1).astype(np.int32)
@@ -22,29 +24,26 @@ def test_sweep_kernels_under_capture(mlpgpu_mod, n, shape):
     s.set_tour(t)
     stream = torch.cuda.Stream()
     assert mlpgpu_mod.lib().mlp_solver_set_stream(s._h, stream.cuda_stream) == 0
+    if total:
+        s.set_total(True)
+    for variant in before:
+        s.set_sweep_kernel(variant)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        graph.capture_begin(capture_error_mode="thread_local")
+        try:
+            if inside is not None:  # no search ran yet: there is no graph to drop during the capture
+                s.set_sweep_kernel(inside)
+            s.sweep(31, 2)
+        finally:
+            graph.capture_end()
+        graph.replay()
+    torch.cuda.synchronize()
+    if total:
+        s.set_total(False)
     want_tour, want = oracle.dvnd(t, D, True, max_iters=12)
-    graphs = []
-    for before, inside in [(1, None), (0, None), (None, 1), (None, 0), (1, None)]:
-        if before is not None:
-            s.set_sweep_kernel(before)
-        torch.cuda.synchronize()
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.stream(stream):
-            graph.capture_begin(capture_error_mode="thread_local")
-            try:
-                if inside is not None:
-                    s.set_sweep_kernel(inside)
-                s.sweep(31, 2)
-            finally:
-                graph.capture_end()
-            graph.replay()
-        torch.cuda.synchronize()
-        graphs.append(graph)
-        s.set_tour(t)
-        st = s.dvnd(max_iters=12)
-        assert np.array_equal(s.tour(), want_tour) and st["cost"] == want["cost"] and st["moves"] == want["moves"]
-        s.set_tour(t)
-    s.set_total(True)
-    s.set_total(False)
+    s.set_tour(t)
     st = s.dvnd(max_iters=12)
-    assert np.array_equal(s.tour(), want_tour) and st["cost"] == want["cost"]
+    assert np.array_equal(s.tour(), want_tour)
+    assert all(st[k] == want[k] for k in ("cost", "iterations", "moves", "evals"))

@@ -250,13 +250,21 @@ MLP_API int mlp_solver_set_tour(mlp_solver_t s, const int32_t* tour, int32_t len
   return s->set->prepare(true);
 }
 
+MLP_API int mlp_problem_set_start_rows(mlp_problem_t h, int32_t mode) {
+  Problem* p = reinterpret_cast<Problem*>(h);
+  if (!p) return arg_error("null problem");
+  if (mode < kStartRowsAuto || mode > kStartRowsUnsorted)
+    return arg_error("start rows must be 0 (automatic), 1 (ordered) or 2 (unsorted)");
+  p->start_rows = mode;
+  return kOk;
+}
+
 MLP_API int mlp_solver_random_tour_ties(mlp_solver_t s, uint32_t seed, float alpha, int32_t ties) {
   MLP_RANGE("mlp_solver_random_tour");
   if (!s) return arg_error("null solver");
   MLP_TRY(check_alpha(alpha));
   if (ties < 0 || ties > 1) return arg_error("ties must be 0 (client id) or 1 (the reference's sort)");
-  const std::vector<GraspTask> task{GraspTask{s->prob->dD, s->job->dev.tour, s->prob->n, seed, alpha, ties, 0}};
-  MLP_TRY(build_random_tours(task, s->set->stream()));
+  MLP_TRY(build_random_tours({start_task(s->prob, s->job->dev.tour, seed, alpha, ties)}, s->set->stream()));
   return s->set->prepare(true);
 }
 
@@ -289,8 +297,8 @@ MLP_API int mlp_problem_random_tours_ties(mlp_problem_t h, int32_t count, const 
   MLP_CUDA(cudaMallocAsync(&r.d, sizeof(int32_t) * sz * (size_t)count, r.st), "cudaMallocAsync(tours)");
   std::vector<GraspTask> tasks;
   for (int32_t q = 0; q < count; q++)
-    tasks.push_back(GraspTask{p->dD, r.d + q * sz, p->n, seeds[q], alpha, ties, 0});
-  MLP_TRY(build_random_tours(tasks, r.st));
+    tasks.push_back(start_task(p, r.d + q * sz, seeds[q], alpha, ties));
+  MLP_TRY(build_random_tours(std::move(tasks), r.st));
   MLP_CUDA(cudaMemcpyAsync(tours, r.d, sizeof(int32_t) * sz * (size_t)count, cudaMemcpyDeviceToHost, r.st),
            "copy tours");
   MLP_CUDA(cudaStreamSynchronize(r.st), "copy tours");
@@ -839,14 +847,14 @@ static int batch_upload(mlp_batch* b) {
     Job* j = b->jobs[q].get();
     if (b->tours[q].empty()) {
       const mlp_batch::RandomStart& rs = b->random_start[q];
-      tasks.push_back(GraspTask{j->prob->dD, j->dev.tour, j->prob->n, rs.seed, rs.alpha, rs.ties, 0});
+      tasks.push_back(start_task(j->prob, j->dev.tour, rs.seed, rs.alpha, rs.ties));
       continue;
     }
     MLP_CUDA(cudaMemcpyAsync(j->dev.tour, b->tours[q].data(), sizeof(int32_t) * b->tours[q].size(),
                              cudaMemcpyHostToDevice, b->stream),
              "copy tour");
   }
-  MLP_TRY(build_random_tours(tasks, b->stream));
+  MLP_TRY(build_random_tours(std::move(tasks), b->stream));
   return b->set->prepare(true);
 }
 

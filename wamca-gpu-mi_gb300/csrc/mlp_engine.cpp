@@ -482,7 +482,12 @@ int check_alpha(float alpha) {
   return kOk;
 }
 
-int build_random_tours(const std::vector<GraspTask>& tasks, cudaStream_t stream) {
+GraspTask start_task(const Problem* p, int32_t* tour, uint32_t seed, float alpha, int ties) {
+  const int32_t kind = ties ? kGraspRef : p->start_rows == kStartRowsUnsorted ? kGraspSelect : kGraspRows;
+  return GraspTask{p->dD, tour, p->n, seed, alpha, kind, 0};
+}
+
+int build_random_tours(std::vector<GraspTask> tasks, cudaStream_t stream) {
   if (tasks.empty()) return kOk;
   struct Buffers {  // stream-ordered: no device-wide synchronisation
     cudaStream_t st;
@@ -496,49 +501,45 @@ int build_random_tours(const std::vector<GraspTask>& tasks, cudaStream_t stream)
         if (p) cudaFreeAsync(p, st);
     }
   } b{stream};
-  // Canonical-tie tasks first, then the reference-tie ones (one launch each);
-  // the former share one set of ordered rows per distance matrix, the latter
-  // above kGraspRefSmemN nodes get 2n words of scratch.
-  std::vector<GraspTask> order;
+  // One launch a kind.  Starts over ordered rows share one set of them per
+  // distance matrix; the reference's order above kGraspRefSmemN nodes takes 2n
+  // words of scratch a start.
+  std::stable_sort(tasks.begin(), tasks.end(), [](const GraspTask& x, const GraspTask& y) { return x.kind < y.kind; });
   std::vector<GraspSortJob> sorts;
   std::map<const int32_t*, int64_t> rows_of;
   int64_t words = 0, entries = 0, nrows = 0;
-  int max_n = 0;
-  for (int pass = 0; pass < 2; pass++)
-    for (GraspTask t : tasks) {
-      if (t.n < 1 || t.n > kMaxSize - 1 || !t.D || !t.tour || t.ties < 0 || t.ties > 1) {
-        set_error("constructor task out of range");
-        return kErrArg;
-      }
-      if (t.ties != pass) continue;
-      t.scratch = 0;
-      if (!t.ties) {
-        const auto at = rows_of.emplace(t.D, entries);
-        if (at.second) {
-          sorts.push_back(GraspSortJob{t.D, entries, nrows, t.n, 0});
-          entries += (int64_t)t.n * t.n;
-          nrows += t.n;
-          max_n = std::max(max_n, t.n);
-        }
-        t.scratch = at.first->second;
-      } else if (t.n > kGraspRefSmemN) {
-        t.scratch = words;
-        words += 2 * (int64_t)t.n;
-      }
-      order.push_back(t);
+  int max_n = 0, count[kGraspKinds] = {};
+  for (GraspTask& t : tasks) {
+    if (t.n < 1 || t.n > kMaxSize - 1 || !t.D || !t.tour || t.kind < 0 || t.kind >= kGraspKinds) {
+      set_error("constructor task out of range");
+      return kErrArg;
     }
-  int ncanon = 0;
-  while (ncanon < (int)order.size() && order[ncanon].ties == 0) ncanon++;
-  MLP_CUDA(cudaMallocAsync(&b.tasks, sizeof(GraspTask) * order.size(), stream), "cudaMallocAsync(constructor tasks)");
+    count[t.kind]++;
+    t.scratch = 0;
+    if (t.kind == kGraspRows) {
+      const auto at = rows_of.emplace(t.D, entries);
+      if (at.second) {
+        sorts.push_back(GraspSortJob{t.D, entries, nrows, t.n, 0});
+        entries += (int64_t)t.n * t.n;
+        nrows += t.n;
+        max_n = std::max(max_n, t.n);
+      }
+      t.scratch = at.first->second;
+    } else if (t.kind == kGraspRef && t.n > kGraspRefSmemN) {
+      t.scratch = words;
+      words += 2 * (int64_t)t.n;
+    }
+  }
+  MLP_CUDA(cudaMallocAsync(&b.tasks, sizeof(GraspTask) * tasks.size(), stream), "cudaMallocAsync(constructor tasks)");
   MLP_CUDA(cudaMallocAsync(&b.err, sizeof(int), stream), "cudaMallocAsync(constructor flag)");
   if (words > 0)
     MLP_CUDA(cudaMallocAsync(&b.scratch, sizeof(uint32_t) * (size_t)words, stream),
              "cudaMallocAsync(constructor scratch)");
-  MLP_CUDA(cudaMemcpyAsync(b.tasks, order.data(), sizeof(GraspTask) * order.size(), cudaMemcpyHostToDevice,
+  MLP_CUDA(cudaMemcpyAsync(b.tasks, tasks.data(), sizeof(GraspTask) * tasks.size(), cudaMemcpyHostToDevice,
                            stream),
            "copy constructor tasks");
   MLP_CUDA(cudaMemsetAsync(b.err, 0, sizeof(int), stream), "memset(constructor flag)");
-  if (ncanon > 0) {
+  if (count[kGraspRows] > 0) {
     // Without room for the ordered rows, or for their sort's jobs, the starts
     // select from unsorted ones.
     if (cudaMallocAsync(&b.sorts, sizeof(GraspSortJob) * sorts.size(), stream) != cudaSuccess) {
@@ -552,9 +553,13 @@ int build_random_tours(const std::vector<GraspTask>& tasks, cudaStream_t stream)
                "copy constructor rows");
       MLP_CUDA(launch_grasp_sort(b.sorts, (int)sorts.size(), nrows, max_n, b.table, stream), "constructor rows kernel");
     }
-    MLP_CUDA(launch_grasp(b.tasks, ncanon, max_n, b.table, b.err, stream), "constructor kernel");
+    MLP_CUDA(launch_grasp(b.tasks, count[kGraspRows], max_n, b.table, b.err, stream), "constructor kernel");
   }
-  MLP_CUDA(launch_grasp_ref(b.tasks + ncanon, (int)order.size() - ncanon, b.scratch, stream), "constructor kernel");
+  const GraspTask* at = b.tasks + count[kGraspRows];
+  if (count[kGraspSelect] > 0)
+    MLP_CUDA(launch_grasp(at, count[kGraspSelect], 0, nullptr, b.err, stream), "constructor kernel");
+  at += count[kGraspSelect];
+  MLP_CUDA(launch_grasp_ref(at, count[kGraspRef], b.scratch, stream), "constructor kernel");
   int herr = 0;
   MLP_CUDA(cudaMemcpyAsync(&herr, b.err, sizeof(int), cudaMemcpyDeviceToHost, stream), "read constructor flag");
   MLP_CUDA(cudaStreamSynchronize(stream), "constructor");

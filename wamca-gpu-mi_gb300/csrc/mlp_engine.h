@@ -42,6 +42,8 @@ void set_error(const std::string& msg);
 const char* last_error();
 int cuda_status(cudaError_t e, const char* what);
 
+enum : int { kStartRowsAuto = 0, kStartRowsOrdered = 1, kStartRowsUnsorted = 2 };
+
 struct Problem {
   int n = 0;
   int size = 0;
@@ -52,6 +54,7 @@ struct Problem {
   int32_t* dD = nullptr;  // n x n
   int32_t* dX = nullptr;  // node coordinates (optional)
   int32_t* dY = nullptr;
+  int start_rows = kStartRowsAuto;  // how canonical starts are built from its distances
   std::vector<int32_t> hx, hy;
   std::string name;
   cudaStream_t alloc_stream = nullptr;  // non-null: stream-ordered allocation
@@ -259,7 +262,9 @@ class JobSet {
 // Start tours of MLSolution::random built on the device (mlp_grasp.cu), one
 // per task, written to the tasks' device tours; waits for the stream and
 // reports a failed internal check.
-int build_random_tours(const std::vector<GraspTask>& tasks, cudaStream_t stream);
+int build_random_tours(std::vector<GraspTask> tasks, cudaStream_t stream);
+// The task of one start (ties as in the C-ABI).
+GraspTask start_task(const Problem* p, int32_t* tour, uint32_t seed, float alpha, int ties);
 // alpha of the constructor must lie in [0, 1].
 int check_alpha(float alpha);
 

@@ -147,18 +147,20 @@ cudaError_t configure_small();
 cudaError_t launch_dvnd_small(const JobDev* job, int size, bool wide, int64_t limit, cudaStream_t s);
 // MLSolution::random on the device (mlp_grasp.cu): one start per task, its
 // n + 1 entries written to `tour` (device), MTRandom seeded with `seed`;
-// alpha in [0, 1].  ties = 0: equal distances ordered by client id (one warp
-// per start over rows ordered once per call); ties = 1: the reference's own
-// order, its std::sort of the persistent candidate array restated step for
-// step (mlp_refsort.cuh; one warp per start, the sort on one lane).
+// alpha in [0, 1].  Equal distances are ordered by client id, one warp per
+// start, over rows ordered once per call (kGraspRows) or by selection among
+// unsorted ones (kGraspSelect); or (kGraspRef) in the reference's own order, its
+// std::sort of the persistent candidate array restated step for step
+// (mlp_refsort.cuh; one warp per start, the sort on one lane).
+enum : int32_t { kGraspRows = 0, kGraspSelect = 1, kGraspRef = 2, kGraspKinds = 3 };
 struct GraspTask {
   const int32_t* D;  // n x n distances
   int32_t* tour;     // n + 1 entries
   int32_t n;
   uint32_t seed;
   float alpha;
-  int32_t ties;
-  int64_t scratch;   // ties = 0: first entry of D's ordered rows; ties = 1 and n > kGraspRefSmemN: word offset of
+  int32_t kind;
+  int64_t scratch;   // kGraspRows: first entry of D's ordered rows; kGraspRef and n > kGraspRefSmemN: word offset of
                      // 2n words in the scratch buffer
 };
 // The rows of one distance matrix, ordered into table[out ...] by the CTAs
@@ -168,14 +170,13 @@ struct GraspSortJob {
   int64_t out, row0;
   int32_t n, pad;
 };
-constexpr int kGraspRefSmemN = 2048;  // ties = 1: up to this n the candidate arrays stay in shared memory
+constexpr int kGraspRefSmemN = 2048;  // kGraspRef: up to this n the candidate arrays stay in shared memory
 cudaError_t configure_grasp();
 cudaError_t launch_grasp_sort(const GraspSortJob* jobs, int njobs, int64_t nrows, int max_n, uint16_t* table, cudaStream_t s);
-// ties = 0 tasks; table: their ordered rows, or null to select from unsorted
-// ones.  *err (device) counts starts that failed an internal check (none
-// expected).
+// kGraspRows tasks with their ordered rows, or (table = null) kGraspSelect tasks.
+// *err (device) counts starts that failed an internal check (none expected).
 cudaError_t launch_grasp(const GraspTask* tasks, int count, int max_n, const uint16_t* table, int* err, cudaStream_t s);
-// ties = 1 tasks; scratch: see GraspTask::scratch.
+// kGraspRef tasks; scratch: see GraspTask::scratch.
 cudaError_t launch_grasp_ref(const GraspTask* tasks, int count, uint32_t* scratch, cudaStream_t s);
 // Or-opt-k for any k in [1, kMaxOroptK] on one job: the per-block candidates
 // (oropt_blocks(k, size) keys, (delta, ctx) as the sweep's) and the pass over

@@ -145,6 +145,7 @@ def lib() -> C.CDLL:
         "mlp_solver_random_tour_ties": (C.c_int, [vp, C.c_uint32, C.c_float, i32]),
         "mlp_problem_random_tours": (C.c_int, [vp, i32, vp, C.c_float, vp]),
         "mlp_problem_random_tours_ties": (C.c_int, [vp, i32, vp, C.c_float, i32, vp]),
+        "mlp_problem_set_start_rows": (C.c_int, [vp, i32]),
         "mlp_batch_run": (C.c_int, [vp, i32, i32]),
         "mlp_batch_reset": (C.c_int, [vp]),
         "mlp_batch_result": (C.c_int, [vp, i32, vp, i32, P(DvndStats)]),
@@ -268,6 +269,11 @@ class Problem:
         _check(lib().mlp_problem_random_tours_ties(self._h, len(sd), _ptr(sd), C.c_float(alpha), int(ties),
                                                    _ptr(out)))
         return out
+
+    def set_start_rows(self, mode: int) -> None:
+        """How starts with ties=0 are built: 0 automatic (default), 1 from rows
+        ordered once per call, 2 by selection from unsorted rows (identical results)."""
+        _check(lib().mlp_problem_set_start_rows(self._h, mode))
 
     def close(self) -> None:
         if self._h:
