@@ -134,11 +134,39 @@ static int constructor_memory() {
   return 0;
 }
 
+// Rows are ordered where enough starts use them or few are to be ordered, not
+// for a start or two of each of very many matrices.
+static int constructor_rule() {
+  struct Case {
+    int n, matrices, starts;
+    bool rows;
+  };
+  for (const Case c : {Case{60, 1, 1, true}, Case{60, 64, 1, true}, Case{60, 512, 1, true}, Case{60, 1100, 1, false},
+                       Case{60, 2000, 1, false}, Case{60, 1100, 4, true}, Case{300, 512, 1, true}, Case{300, 900, 1, false},
+                       Case{300, 600, 4, true}}) {
+    mlp_batch_t b = nullptr;
+    REQUIRE(mlp_batch_create(0, &b) == 0);
+    std::vector<mlp_problem_t> ps;
+    for (int m = 0; m < c.matrices; m++) {
+      ps.push_back(problem(c.n, 100));
+      for (int q = 0; q < c.starts; q++) REQUIRE(mlp_batch_add_random(b, ps.back(), q, 0.5f, nullptr) == 0);
+    }
+    fake::grasp_table = &fake::calls;
+    REQUIRE(mlp_batch_reset(b) == 0);
+    if ((fake::grasp_table != nullptr) != c.rows) std::fprintf(stderr, "n %d, %d x %d\n", c.n, c.matrices, c.starts);
+    REQUIRE((fake::grasp_table != nullptr) == c.rows);
+    mlp_batch_destroy(b);
+    for (mlp_problem_t p : ps) mlp_problem_destroy(p);
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string check = argc > 1 ? argv[1] : "";
   if (check == "batch_result") return batch_result();
   if (check == "captured_sweeps") return captured_sweeps();
   if (check == "constructor_memory") return constructor_memory();
+  if (check == "constructor_rule") return constructor_rule();
   std::fprintf(stderr, "unknown check\n");
   return 2;
 }

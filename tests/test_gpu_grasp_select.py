@@ -57,3 +57,19 @@ def test_kinds_in_one_call(mlpgpu_mod):
     for j, (t, st) in enumerate(want):
         bt, bst = b.result(j)
         assert np.array_equal(bt, t) and bst["cost"] == st["cost"], j
+
+
+@pytest.mark.parametrize("matrices", [740, 800, 1250])
+def test_many_matrices(mlpgpu_mod, matrices):
+    """Either side of the rule between ordered rows and selection (one start a matrix)."""
+    n, b, want = 24, mlpgpu_mod.Batch(), []
+    for q in range(matrices):
+        x, y = oracle.uniform_instance(n, q)
+        b.add_random(mlpgpu_mod.Problem.from_coords(x, y), q, 0.5)
+        if q % 97 == 0:
+            D = oracle.dist(x, y, True)
+            want.append((q, *oracle.dvnd(oracle.random_tour_canonical(D, q, 0.5), D)))
+    b.run()
+    for q, t, st in want:
+        bt, bst = b.result(q)
+        assert np.array_equal(bt, t) and bst["cost"] == st["cost"]

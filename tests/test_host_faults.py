@@ -38,3 +38,7 @@ def test_sweeps_on_a_capturing_stream(exe):
 
 def test_constructor_memory(exe):
     _run(exe, "constructor_memory")
+
+
+def test_constructor_rule(exe):
+    _run(exe, "constructor_rule")

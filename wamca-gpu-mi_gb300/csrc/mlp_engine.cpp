@@ -11,6 +11,7 @@
 #include <cstring>
 #include <fstream>
 #include <sstream>
+#include <unordered_map>
 
 #include "mlp_kernels.cuh"
 
@@ -482,8 +483,31 @@ int check_alpha(float alpha) {
   return kOk;
 }
 
+// Ordered rows pay for `starts` starts over matrices of `entries` distances in
+// all.  The sort's time goes with the entries; the selection's with the waves of
+// starts that are at work at once (a CTA of 8 on each of 152 SMs) and the largest
+// matrix.  One wave costs as much as sorting 440 to 750 matrices of its size.  Us
+// a call, one start each of 304 / 608 / 1,024 / 1,217 / 2,048 matrices, ordered
+// rows | selection:
+//   n = 100    277 | 525   447 | 542   699 | 554   825 | 892   1,357 | 1,069
+//   n = 200    613 | 1,080   1,109 | 1,143   1,757 | 1,194   2,063 | 2,154   3,382 | 2,368
+//   n = 1000   7,758 | 12,904   14,180 | 12,988   22,979 | 13,032   27,086 | 24,984   44,793 | 25,852
+//   n = 2000   32,213 | 44,513   60,708 | 44,622   99,775 | 44,709   117,898 | 85,449
+// and with two starts each of 1,024 matrices of n = 1000 23,189 | 25,729.  Above
+// 2048 nodes a selecting step gathers its keys from L2 in every pass (4 starts at
+// n = 5000: 15.6 ms | 535).
+static bool start_rows_pay(int max_n, int64_t starts, int64_t entries) {
+  if (max_n > 2048) return true;
+  const int64_t waves = (starts + 8 * 152 - 1) / (8 * 152);
+  const int64_t matrices = max_n <= 128 ? 750 : max_n <= 256 ? 650 : max_n <= 1024 ? 570 : 440;
+  return entries <= matrices * waves * max_n * max_n;
+}
+
 GraspTask start_task(const Problem* p, int32_t* tour, uint32_t seed, float alpha, int ties) {
-  const int32_t kind = ties ? kGraspRef : p->start_rows == kStartRowsUnsorted ? kGraspSelect : kGraspRows;
+  const int32_t kind = ties                                  ? kGraspRef
+                       : p->start_rows == kStartRowsAuto     ? kGraspAuto
+                       : p->start_rows == kStartRowsUnsorted ? kGraspSelect
+                                                             : kGraspRows;
   return GraspTask{p->dD, tour, p->n, seed, alpha, kind, 0};
 }
 
@@ -501,35 +525,57 @@ int build_random_tours(std::vector<GraspTask> tasks, cudaStream_t stream) {
         if (p) cudaFreeAsync(p, st);
     }
   } b{stream};
-  // One launch a kind.  Starts over ordered rows share one set of them per
-  // distance matrix; the reference's order above kGraspRefSmemN nodes takes 2n
-  // words of scratch a start.
-  std::stable_sort(tasks.begin(), tasks.end(), [](const GraspTask& x, const GraspTask& y) { return x.kind < y.kind; });
+  // Starts over ordered rows share one set of them per distance matrix; the
+  // reference's order above kGraspRefSmemN nodes takes 2n words of scratch a start.
   std::vector<GraspSortJob> sorts;
-  std::map<const int32_t*, int64_t> rows_of;
-  int64_t words = 0, entries = 0, nrows = 0;
+  std::unordered_map<const int32_t*, int64_t> rows_of;
+  int64_t words = 0, entries = 0, nrows = 0, autos = 0;
   int max_n = 0, count[kGraspKinds] = {};
+  auto order_rows = [&](GraspTask& t) {
+    if (!sorts.empty() && sorts.back().D == t.D) {
+      t.scratch = sorts.back().out;
+      return;
+    }
+    const auto at = rows_of.emplace(t.D, entries);
+    t.scratch = at.first->second;
+    if (!at.second) return;
+    sorts.push_back(GraspSortJob{t.D, entries, nrows, t.n, 0});
+    entries += (int64_t)t.n * t.n;
+    nrows += t.n;
+    max_n = std::max(max_n, t.n);
+  };
   for (GraspTask& t : tasks) {
-    if (t.n < 1 || t.n > kMaxSize - 1 || !t.D || !t.tour || t.kind < 0 || t.kind >= kGraspKinds) {
+    if (t.n < 1 || t.n > kMaxSize - 1 || !t.D || !t.tour || t.kind < kGraspAuto || t.kind >= kGraspKinds) {
       set_error("constructor task out of range");
       return kErrArg;
     }
-    count[t.kind]++;
     t.scratch = 0;
-    if (t.kind == kGraspRows) {
-      const auto at = rows_of.emplace(t.D, entries);
-      if (at.second) {
-        sorts.push_back(GraspSortJob{t.D, entries, nrows, t.n, 0});
-        entries += (int64_t)t.n * t.n;
-        nrows += t.n;
-        max_n = std::max(max_n, t.n);
-      }
-      t.scratch = at.first->second;
+    if (t.kind == kGraspAuto) {
+      autos++;
+      order_rows(t);
+    }
+  }
+  const int32_t kind = start_rows_pay(max_n, autos, entries) ? kGraspRows : kGraspSelect;
+  if (kind == kGraspSelect) {
+    sorts.clear();
+    rows_of.clear();
+    entries = nrows = 0;
+    max_n = 0;
+  }
+  for (GraspTask& t : tasks) {
+    if (t.kind == kGraspAuto) {
+      t.kind = kind;
+    } else if (t.kind == kGraspRows) {
+      order_rows(t);
     } else if (t.kind == kGraspRef && t.n > kGraspRefSmemN) {
       t.scratch = words;
       words += 2 * (int64_t)t.n;
     }
+    count[t.kind]++;
   }
+  // One launch a kind.
+  const auto by_kind = [](const GraspTask& x, const GraspTask& y) { return x.kind < y.kind; };
+  if (!std::is_sorted(tasks.begin(), tasks.end(), by_kind)) std::stable_sort(tasks.begin(), tasks.end(), by_kind);
   MLP_CUDA(cudaMallocAsync(&b.tasks, sizeof(GraspTask) * tasks.size(), stream), "cudaMallocAsync(constructor tasks)");
   MLP_CUDA(cudaMallocAsync(&b.err, sizeof(int), stream), "cudaMallocAsync(constructor flag)");
   if (words > 0)

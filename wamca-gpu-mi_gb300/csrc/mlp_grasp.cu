@@ -25,8 +25,9 @@
 // 9.5 -> 1.23, 2048 starts 18.7 -> 1.66; 4 starts at n = 5000 535 -> 15.6.
 // The sort is bound by its shared-memory passes (23 us at n = 1000), a start by
 // the chain of its steps.
-// The ordered rows take 2 n^2 bytes of scratch; where that cannot be allocated
-// k_grasp_select serves.
+// The ordered rows take 2 n^2 bytes of scratch a matrix; where that cannot be
+// allocated, and for a start or two of each of very many matrices
+// (start_rows_pay), k_grasp_select serves.
 #include <cmath>
 #include <cstdint>
 

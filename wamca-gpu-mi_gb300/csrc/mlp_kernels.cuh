@@ -149,10 +149,11 @@ cudaError_t launch_dvnd_small(const JobDev* job, int size, bool wide, int64_t li
 // n + 1 entries written to `tour` (device), MTRandom seeded with `seed`;
 // alpha in [0, 1].  Equal distances are ordered by client id, one warp per
 // start, over rows ordered once per call (kGraspRows) or by selection among
-// unsorted ones (kGraspSelect); or (kGraspRef) in the reference's own order, its
+// unsorted ones (kGraspSelect), whichever pays (kGraspAuto, before the launches);
+// or (kGraspRef) in the reference's own order, its
 // std::sort of the persistent candidate array restated step for step
 // (mlp_refsort.cuh; one warp per start, the sort on one lane).
-enum : int32_t { kGraspRows = 0, kGraspSelect = 1, kGraspRef = 2, kGraspKinds = 3 };
+enum : int32_t { kGraspAuto = -1, kGraspRows = 0, kGraspSelect = 1, kGraspRef = 2, kGraspKinds = 3 };
 struct GraspTask {
   const int32_t* D;  // n x n distances
   int32_t* tour;     // n + 1 entries
