@@ -143,7 +143,7 @@ MLP_API int mlp_solver_set_unroll(mlp_solver_t s, int32_t iterations);
  * identical; the switch exists for measurement and testing. */
 MLP_API int mlp_solver_set_sweep_kernel(mlp_solver_t s, int32_t variant);
 /* Merge kernel of the solver's iterations (as mlp_batch_set_merge_mode; the
- * default for one search is one CTA up to about 2,038 nodes, then the six-CTA
+ * default for one search is one CTA up to 1,999 nodes, then the six-CTA
  * cluster).  Every mode gives the same results. */
 MLP_API int mlp_solver_set_merge_mode(mlp_solver_t s, int32_t mode);
 /* Candidate mode of every later pass / DVND of this solver.  0 (default): one
@@ -299,7 +299,7 @@ MLP_API int mlp_batch_result(mlp_batch_t b, int32_t job, int32_t* tour, int32_t 
                              mlp_dvnd_stats_t* stats);
 MLP_API int mlp_batch_set_tile_shape(mlp_batch_t b, int32_t shape);
 /* Merge kernel of the batch's iterations: 0 = automatic (one CTA per job up
- * to 1,045 nodes and for 16 jobs or more, otherwise a six-CTA cluster per job), 1 = cluster, 2 = one
+ * to 1,093 nodes and for 16 jobs or more, otherwise a six-CTA cluster per job), 1 = cluster, 2 = one
  * CTA per job.  Every mode gives the same results. */
 MLP_API int mlp_batch_set_merge_mode(mlp_batch_t b, int32_t mode);
 /* DVND sweep kernel of the batch's iterations (as mlp_solver_set_sweep_kernel). */

@@ -29,7 +29,9 @@
 namespace mlp {
 namespace {
 
-constexpr int kOneMaxBlocks = 2112;  // most candidates of a neighbourhood
+// Largest tour (positions; see merge_one_serves): a neighbourhood has fewer
+// candidates.
+constexpr int kOneMaxSize = 2000;
 
 // Shared memory (bytes): the stage-3 list, then the candidate lists and swap
 // tables of stage 2, under which the conflict rows, the position map, the old
@@ -215,7 +217,7 @@ __device__ __forceinline__ void swap_tables(int sz, int c, int gtid, int gnt, in
 template <bool WIDE, int NT>
 __device__ __forceinline__ void one_rebuild(const JobDev* J, int sz, const int32_t* t, int32_t* w_s, const int32_t* src) {
   using C = typename Arith<WIDE>::C;
-  constexpr int PER = (kOneMaxBlocks + 8 + NT - 1) / NT, nw = NT / 32;
+  constexpr int PER = (kOneMaxSize + 8 + NT - 1) / NT, nw = NT / 32;
   __shared__ C s_w[PER * nw], s_q[PER * nw];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, n = J->n, pad = sz + 8;
   const int32_t* __restrict__ D = J->D;
@@ -369,7 +371,7 @@ __global__ void __launch_bounds__(NT) k_merge_one(const JobDev* __restrict__ job
   if (tid < (int)(sizeof(JobDev) / 8)) ((uint64_t*)&s_job)[tid] = ((const uint64_t*)Jg)[tid];
   // The current tour, in registers until stage 2 is over.
   const int32_t* tour = Jg->tour;
-  constexpr int kTourPer = (kOneMaxBlocks + 8 + NT - 1) / NT;
+  constexpr int kTourPer = (kOneMaxSize + 8 + NT - 1) / NT;
   int32_t mine[kTourPer];
 #pragma unroll
   for (int u = 0; u < kTourPer; u++) mine[u] = tid + u * nt < sz ? tour[tid + u * nt] : 0;
@@ -429,7 +431,7 @@ __global__ void __launch_bounds__(NT) k_merge_one(const JobDev* __restrict__ job
         else swap_tables<12>(sz, c, gtid, gnt, 1, tab, lkey, lab, list);
       } else {
         uint64_t* gm = s_gmin[nb - 1];
-        constexpr int kGroupPer = (kOneMaxBlocks + 32 * kIntWarps - 1) / (32 * kIntWarps);
+        constexpr int kGroupPer = (kOneMaxSize + 32 * kIntWarps - 1) / (32 * kIntWarps);
         if (c <= 128) {
           if (gtid < 32) {
             if (c <= 32) interval_greedy<1>(nb, c, gtid, 1, 0, gm, lkey, lab, list);
@@ -524,7 +526,7 @@ cudaError_t one_launch(const JobDev* jobs, int njobs, int threads, size_t smem, 
 int merge_one_max_size() {
   static const int cached = [] {
     int sz = 8;
-    while (sz < kMaxSize && nb_blocks(2, sz + 1) <= kOneMaxBlocks && OneLayout(sz + 1).total <= kOneSmem) sz++;
+    while (sz < kOneMaxSize && OneLayout(sz + 1).total <= kOneSmem) sz++;
     return sz;
   }();
   return cached;
@@ -542,12 +544,22 @@ cudaError_t configure_merge_one() {
   return e;
 }
 
-// Where this merge serves: one search up to merge_one_max_size(), more than one
-// while two of its CTAs fit an SM (n = 1045).  Larger merges of several
-// searches take an SM's whole shared memory, which then has to be split anew
-// between the sweep's CTAs and its L1 cache: 64 searches of n in [1900, 2000]
-// 286 -> 342 ms (20 of them 95 -> 103), while the merge alone is faster (93 ->
-// 55 us).
+// Where this merge serves, all limits in positions.  One search: up to 2,000
+// (merge_one_max_size(); 2,115 would fit its shared memory).  Us an iteration,
+// this merge | the cluster's: n = 1100 22.6 | 24.5, 1500 27.0 | 28.3, 1700 29.2 |
+// 29.8, 1900 33.3 | 33.3, 1999 34.2 | 34.5; 64-bit 1100 23.5 | 25.1, 1500 36.5 |
+// 39.9, 1700 40.8 | 41.1, 1999 42.8 | 43.1.  The longer the lists, the less the
+// cluster's hand-off counts: built for 2,115, with a third position a thread, it
+// took 36.0 | 35.9 at 2050 and 37.5 | 37.1 at 2114, 64-bit 44.8 | 44.2 and 45.8 |
+// 45.0.
+// Several searches: while the layout takes at most 113 KB (1,094 positions).  Its
+// CTAs run one an SM at any size (1,024 threads of 64 registers); of larger
+// layouts the sweep seems to suffer, whose CTAs and L1 cache share what a merge
+// leaves of an SM (not measured apart).  Ms a set, this merge | cluster |
+// k_merge_solo: 24 of n in [1046, 1093] 26.4 | 28.4 | 34.8,
+// 256 of them 195 | 233 | 209, 256 of [900, 1000] 155 | 188 | 159; but 64 of
+// [1900, 2000] 342 where k_merge_solo takes 286, and 20 of them 103 | . | 95, while
+// the merge alone is faster (93 -> 55 us).  Between, nothing was measured.
 bool merge_one_serves(int njobs, int max_size) {
   if (max_size > merge_one_max_size()) return false;
   return njobs == 1 || OneLayout(max_size).total <= 113u * 1024u;
