@@ -142,6 +142,12 @@ MLP_API int mlp_solver_set_unroll(mlp_solver_t s, int32_t iterations);
  * evaluate all five neighbourhoods), 0 the general fused sweep.  Results are
  * identical; the switch exists for measurement and testing. */
 MLP_API int mlp_solver_set_sweep_kernel(mlp_solver_t s, int32_t variant);
+/* The one-launch search of small tours (no counterpart in the reference), for
+ * measurement and testing: its CTAs (0, the default: 16, or 8 where a cluster of
+ * 16 cannot be placed; 8; 16; -1: never, the iterated kernels run), and how often
+ * a wait for distance rows is polled before the search ends with MLP_ERR_STATE
+ * (-1, the default: 2^20 times, a second or more).  Results are identical. */
+MLP_API int mlp_solver_set_small_search(mlp_solver_t s, int32_t ctas, int32_t polls);
 /* Merge kernel of the solver's iterations (as mlp_batch_set_merge_mode; the
  * default for one search is one CTA up to 1,999 nodes, then the six-CTA
  * cluster).  Every mode gives the same results. */

@@ -98,14 +98,14 @@ size_t merge_ws_bytes(int) { return 1024; }
 int merge_smem_max_size() { return 2000; }
 int solo_smem_max_size() { return 1500; }
 size_t oropt_pass_scratch_bytes(int size, int) { return 64 * (size_t)size; }
-bool small_fits(int size) { return size <= 385; }
+bool small_fits(int size, int) { return size <= 385; }
 bool merge_one_serves(int njobs, int max_size) { return max_size <= (njobs == 1 ? 2000 : 1000); }
 cudaError_t configure_merge(size_t) { return fake::call(__func__); }
 cudaError_t configure_merge_one() { return fake::call(__func__); }
 cudaError_t configure_small() { return fake::call(__func__); }
 cudaError_t launch_ads(const JobDev*, const int32_t*, const int32_t*, uint32_t*, int, int, cudaStream_t, uint32_t*, int) { return fake::call(__func__); }
 cudaError_t launch_dist(const int32_t*, const int32_t*, int, int, int32_t*, int32_t*, cudaStream_t) { return fake::call(__func__); }
-cudaError_t launch_dvnd_small(const JobDev*, int, bool, int64_t, cudaStream_t) { return fake::call(__func__); }
+cudaError_t launch_dvnd_small(const JobDev*, int, bool, int64_t, int, int, cudaStream_t) { return fake::call(__func__); }
 cudaError_t launch_grasp(const GraspTask*, int, int, const uint16_t* table, int*, cudaStream_t) {
   fake::grasp_table = table;
   return fake::call(__func__);

@@ -32,13 +32,12 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                : "memory");
 }
 
-// Waits for phase `parity` of the barrier, at most kMbarTries polls suspended
-// for a microsecond or so each (far longer than any copy takes); false if it
-// did not complete.
-constexpr int kMbarTries = 1 << 20;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+// Waits for phase `parity` of the barrier, at most `tries` polls suspended for
+// a microsecond or so each (kMbarTries: far longer than any copy takes); false
+// if it did not complete.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int tries) {
   const uint32_t a = smem_addr(bar);
-  for (int q = 0; q < kMbarTries; q++) {
+  for (int q = 0; q < tries; q++) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"

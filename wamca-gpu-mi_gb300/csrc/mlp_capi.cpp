@@ -235,6 +235,14 @@ MLP_API int mlp_solver_set_sweep_kernel(mlp_solver_t s, int32_t variant) {
   return s->set->set_sweep_kernel(variant);
 }
 
+MLP_API int mlp_solver_set_small_search(mlp_solver_t s, int32_t ctas, int32_t polls) {
+  if (!s) return arg_error("null solver");
+  if ((ctas != -1 && ctas != 0 && ctas != 8 && ctas != 16) || polls < -1)
+    return arg_error("small search: ctas must be -1, 0, 8 or 16, polls at least -1");
+  s->set->set_small_search(ctas, polls < 0 ? kMbarTries : polls);
+  return kOk;
+}
+
 MLP_API int mlp_solver_set_total(mlp_solver_t s, int32_t on) {
   if (!s) return arg_error("null solver");
   return s->set->set_total(on != 0);

@@ -1051,7 +1051,7 @@ bool JobSet::small_search() const {
   if (all_jobs_.size() != 1 || total_ || mask_ != 0x1f || merge_mode_ != kMergeAuto || sweep_variant_ != 1) return false;
   const Job* j = all_jobs_[0];
   if (j->dev.flags & kFlagRecordMoves) return false;
-  return small_fits(j->size) && (!wide_ || fits32(j));
+  return small_ctas_ >= 0 && small_fits(j->size, small_ctas_) && (!wide_ || fits32(j));
 }
 
 int JobSet::enqueue_device_loop(int max_iters) {
@@ -1068,7 +1068,7 @@ int JobSet::enqueue_device_loop(int max_iters) {
     if (st != kOk) return st;
   }
   if (small_search()) {
-    MLP_CUDA(launch_dvnd_small(djobs_, max_size_, wide_, max_iters, stream_), "search kernel");
+    MLP_CUDA(launch_dvnd_small(djobs_, max_size_, wide_, max_iters, small_ctas_, small_polls_, stream_), "search kernel");
     return kOk;
   }
   const int unroll = kDeviceLoopBody;

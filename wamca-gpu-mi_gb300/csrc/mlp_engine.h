@@ -196,6 +196,12 @@ class JobSet {
   // that evaluate all five neighbourhoods (k_sweep_dvnd), 0 the general
   // kernel everywhere.  Both give identical candidates.
   int set_sweep_kernel(int variant);
+  // The one-launch search's CTAs (0: as many as fit, 8, 16; -1: not taken) and
+  // its polls of a wait for copied rows.
+  void set_small_search(int ctas, int polls) {
+    small_ctas_ = ctas;
+    small_polls_ = polls;
+  }
   int sweep_kernel_variant() const { return sweep_variant_; }
 
  private:
@@ -243,6 +249,7 @@ class JobSet {
   int merge_mode_ = 0;
   bool total_ = false;
   int sweep_variant_ = 1;
+  int small_ctas_ = 0, small_polls_ = kMbarTries;
   int shape_user_ = -1;  // tile shape to restore when TOTAL mode ends
   JobDev* djobs_ = nullptr;
   TileList lists_[2];

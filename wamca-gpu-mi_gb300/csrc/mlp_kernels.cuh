@@ -142,9 +142,13 @@ cudaError_t configure_total();
 // A whole DVND (all five neighbourhoods, 32-bit deltas) of one small search in
 // one launch (mlp_small.cu): the job's tour, arrays and statistics afterwards
 // are those of the iterated sweep and merge.
-bool small_fits(int size);
+// small_fits: `ctas` = 0 asks for the largest cluster that the device places, 8
+// or 16 for that one.  polls: of each wait for copied distance rows, after which
+// the search ends with an error.
+constexpr int kMbarTries = 1 << 20;
+bool small_fits(int size, int ctas);
 cudaError_t configure_small();
-cudaError_t launch_dvnd_small(const JobDev* job, int size, bool wide, int64_t limit, cudaStream_t s);
+cudaError_t launch_dvnd_small(const JobDev* job, int size, bool wide, int64_t limit, int ctas, int polls, cudaStream_t s);
 // MLSolution::random on the device (mlp_grasp.cu): one start per task, its
 // n + 1 entries written to `tour` (device), MTRandom seeded with `seed`;
 // alpha in [0, 1].  Equal distances are ordered by client id, one warp per

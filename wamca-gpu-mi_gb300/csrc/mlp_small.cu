@@ -272,7 +272,7 @@ __device__ __forceinline__ void small_intervals(int nb, int c, const uint64_t* l
 
 // One search to its local optimum (or `limit` sweeps), by one cluster.
 template <bool WIDE, bool RESIDENT>
-__global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __restrict__ J, int64_t limit) {
+__global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __restrict__ J, int64_t limit, int polls) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_cnt[kNumNb], s_m3, s_ns, s_ntiles;
   __shared__ uint32_t s_scan[2][32];
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __re
     tour0[p] = p < sz ? J->tour[p] : 0;
     tour0[tstride + p] = 0;
   }
-  if (tid == 0) s_ntiles = 0;
+  if (tid == 0) s_ntiles = ctl[1] = 0;
   __syncthreads();
   if (merger) {
     for (int p = tid; p < sz; p += nt) src[p] = p;
@@ -328,7 +328,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __re
     }
   }
   int64_t sweeps = 0, moves = 0, iters = 0, last = 0;
-  bool converged = false, lost = false;
+  bool converged = false, lost = false;  // lost: this CTA's rows of an iteration did not arrive
+  uint32_t lost_phase = 0;
   int cur = 0;
   cluster.sync();
   for (;;) {
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __re
         // The distance rows of this CTA's blocks (positions past the tour's
         // end: its last row again), the 16-byte words that hold each (D's
         // allocation extends 16 bytes past the last row).
-        if (tid < myblocks * (B + 3)) {
+        if (!lost && tid < myblocks * (B + 3)) {
           const int lb = tid / (B + 3), p = min((lb * sweepers + sw) * B + tid % (B + 3), sz - 1);
           const uintptr_t a = reinterpret_cast<uintptr_t>(J->D + (size_t)t[p] * n);
           const uint32_t off = (uint32_t)(a & 15), bytes = (off + 4u * (uint32_t)n + 15u) & ~15u;
@@ -393,14 +394,17 @@ __global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __re
       }
       __syncthreads();
       // ---- this CTA's tiles ----
+      bool here = !lost;
       if constexpr (!RESIDENT) {
-        // Bounded: if the rows do not arrive the search ends with an error.
-        if (!lost && !mbar_wait(bar, (uint32_t)(sweeps & 1))) {
-          lost = true;
+        // Bounded: a CTA whose rows do not arrive copies and sweeps no more, and
+        // the search ends with an error.
+        if (here && !mbar_wait(bar, (uint32_t)(sweeps & 1), polls)) {
+          here = false;
+          ctl[1] = 1;
           J->stats[kStatError] = 6;
         }
       }
-      const int ntiles = lost ? 0 : s_ntiles;
+      const int ntiles = here ? s_ntiles : 0;
       for (int k = wid; k < ntiles; k += nw) {
         const uint32_t tl = tiles[k];
         const int rs = (int)(tl & 511u), L0 = (int)((tl >> 9) & 511u);
@@ -500,9 +504,21 @@ __global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __re
     }
     cluster.sync();  // the next tour
     cur ^= 1;
-    if (!*ctl) break;
+    if constexpr (RESIDENT) {
+      if (!*ctl) break;
+    } else {
+      const uint64_t both = *reinterpret_cast<volatile uint64_t*>(smem);  // go, rows lost
+      if (!lost && (both >> 32) != 0) {
+        lost = true;
+        lost_phase = (uint32_t)((sweeps - 1) & 1);
+      }
+      if ((uint32_t)both == 0) break;
+    }
   }
-  if (!merger) return;
+  if (!merger) {
+    if (lost) mbar_wait(bar, lost_phase, kMbarTries);  // a CTA outlives its copies in flight
+    return;
+  }
   // ---- the job's arrays and statistics as the two-kernel loop leaves them ----
   const int32_t* t = tour0 + cur * tstride;
   for (int p = tid; p < sz; p += nt) J->tour[p] = t[p];
@@ -519,7 +535,6 @@ __global__ void __launch_bounds__(kSmallThreads) k_dvnd_small(const JobDev* __re
   cta_prepare<WIDE>(J, t, src);  // the position map is dead: w staging
 }
 
-constexpr int kSmallCluster = 16;
 constexpr uint32_t kSmallSmem = 227 * 1024 - 4096;  // room for the static shared memory
 
 uint32_t small_smem(int size, int cluster, bool resident) {
@@ -528,7 +543,7 @@ uint32_t small_smem(int size, int cluster, bool resident) {
   return a > b ? a : b;
 }
 
-void (*small_kernel(bool wide, bool resident))(const JobDev*, int64_t) {
+void (*small_kernel(bool wide, bool resident))(const JobDev*, int64_t, int) {
   if (wide) return resident ? k_dvnd_small<true, true> : k_dvnd_small<true, false>;
   return resident ? k_dvnd_small<false, true> : k_dvnd_small<false, false>;
 }
@@ -548,36 +563,36 @@ cudaLaunchConfig_t small_config(int cluster, uint32_t smem, cudaLaunchAttribute*
   return cfg;
 }
 
-// CTAs of a cluster: kSmallCluster where the device places that many (a
-// non-portable size), else 8 (queried once, with the most shared memory).
+// CTAs of a cluster: 16 where the device places that many (a non-portable
+// size), else 8 (queried once, with the most shared memory).
 int small_cluster() {
   static const int cluster = [] {
     cudaLaunchAttribute attr;
-    const cudaLaunchConfig_t cfg = small_config(kSmallCluster, kSmallSmem, &attr, 0);
+    const cudaLaunchConfig_t cfg = small_config(16, kSmallSmem, &attr, 0);
     int c = 0;
     if (configure_small() != cudaSuccess || cudaOccupancyMaxActiveClusters(&c, small_kernel(false, true), &cfg) != cudaSuccess) {
       cudaGetLastError();
       c = 0;
     }
-    return c >= 1 ? kSmallCluster : 8;
+    return c >= 1 ? 16 : 8;
   }();
   return cluster;
 }
 
 }  // namespace
 
-bool small_fits(int size) {
-  const int n = size - 1, cl = small_cluster();
-  if (n < 5 || size > kSmallMaxSize) return false;
+bool small_fits(int size, int ctas) {
+  const int n = size - 1, cl = ctas ? ctas : small_cluster();
+  if (n < 5 || size > kSmallMaxSize || cl > small_cluster()) return false;
   return SmallLayout::slots(size, cl - 1) <= kSmallSlots && small_smem(size, cl, false) <= kSmallSmem;
 }
 
-cudaError_t launch_dvnd_small(const JobDev* job, int size, bool wide, int64_t limit, cudaStream_t s) {
-  const int cl = small_cluster();
+cudaError_t launch_dvnd_small(const JobDev* job, int size, bool wide, int64_t limit, int ctas, int polls, cudaStream_t s) {
+  const int cl = ctas ? ctas : small_cluster();
   const bool resident = small_smem(size, cl, true) <= kSmallSmem;
   cudaLaunchAttribute attr;
   const cudaLaunchConfig_t cfg = small_config(cl, small_smem(size, cl, resident), &attr, s);
-  return cudaLaunchKernelEx(&cfg, small_kernel(wide, resident), job, limit);
+  return cudaLaunchKernelEx(&cfg, small_kernel(wide, resident), job, limit, polls);
 }
 
 cudaError_t configure_small() {

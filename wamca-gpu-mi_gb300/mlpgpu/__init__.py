@@ -146,6 +146,7 @@ def lib() -> C.CDLL:
         "mlp_problem_random_tours": (C.c_int, [vp, i32, vp, C.c_float, vp]),
         "mlp_problem_random_tours_ties": (C.c_int, [vp, i32, vp, C.c_float, i32, vp]),
         "mlp_problem_set_start_rows": (C.c_int, [vp, i32]),
+        "mlp_solver_set_small_search": (C.c_int, [vp, i32, i32]),
         "mlp_batch_run": (C.c_int, [vp, i32, i32]),
         "mlp_batch_reset": (C.c_int, [vp]),
         "mlp_batch_result": (C.c_int, [vp, i32, vp, i32, P(DvndStats)]),
@@ -324,6 +325,11 @@ class Solver:
         """DVND sweep kernel: 1 (default) row/column term tables, 0 the
         general fused sweep; identical results."""
         _check(lib().mlp_solver_set_sweep_kernel(self._h, variant))
+
+    def set_small_search(self, ctas: int = 0, polls: int = -1) -> None:
+        """CTAs of the one-launch search (0 automatic, 8, 16; -1 never) and the
+        polls of its waits (-1: the default)."""
+        _check(lib().mlp_solver_set_small_search(self._h, ctas, polls))
 
     def set_merge_mode(self, mode: int) -> None:
         """0 automatic, 1 six-CTA cluster, 2 one CTA; identical results."""
