@@ -161,12 +161,34 @@ static int constructor_rule() {
   return 0;
 }
 
+// Without the one-launch search (its kernels refused by the device) the iterated
+// kernels serve; nothing is refused.
+static int no_small_search() {
+  const int n = 50;
+  mlp_problem_t p = problem(n, 100);
+  const std::vector<int32_t> t = tour(n);
+  for (bool refused : {false, true}) {
+    mlp_solver_t s = nullptr;
+    if (refused) fake::fail("configure_small", cudaErrorInvalidValue);
+    REQUIRE(p && mlp_solver_create(p, 0, &s) == 0);
+    fake::fails.clear();
+    REQUIRE(mlp_solver_set_tour(s, t.data(), n + 1) == 0);
+    fake::calls.clear();
+    REQUIRE(mlp_solver_dvnd_async(s, MLP_NB_ALL, 5) == 0);
+    REQUIRE(fake::calls["launch_dvnd_small"] == (refused ? 0 : 1) && fake::calls["launch_merge_one"] == (refused ? 5 : 0));
+    mlp_solver_destroy(s);
+  }
+  mlp_problem_destroy(p);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string check = argc > 1 ? argv[1] : "";
   if (check == "batch_result") return batch_result();
   if (check == "captured_sweeps") return captured_sweeps();
   if (check == "constructor_memory") return constructor_memory();
   if (check == "constructor_rule") return constructor_rule();
+  if (check == "no_small_search") return no_small_search();
   std::fprintf(stderr, "unknown check\n");
   return 2;
 }

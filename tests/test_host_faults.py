@@ -42,3 +42,7 @@ def test_constructor_memory(exe):
 
 def test_constructor_rule(exe):
     _run(exe, "constructor_rule")
+
+
+def test_without_the_small_search(exe):
+    _run(exe, "no_small_search")

@@ -665,7 +665,10 @@ int JobSet::init() {
     }
   }
   MLP_CUDA(configure_merge(merge_smem_ ? merge_smem_bytes(max_size_) : 0), "configure merge");
-  MLP_CUDA(configure_small(), "configure search");
+  if (configure_small() != cudaSuccess) {  // the iterated kernels serve
+    cudaGetLastError();
+    small_ctas_ = -1;
+  }
   MLP_CUDA(configure_merge_one(), "configure merge");
   size_t result = kResultHead + ((size_t)max_size_ + 1) / 2;
   for (const Job* j : jobs_) result = std::max(result, kStatWords + (size_t)j->moves_cap + ((size_t)j->moves_cap + 1) / 2);

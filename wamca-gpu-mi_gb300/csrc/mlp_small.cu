@@ -563,18 +563,22 @@ cudaLaunchConfig_t small_config(int cluster, uint32_t smem, cudaLaunchAttribute*
   return cfg;
 }
 
-// CTAs of a cluster: 16 where the device places that many (a non-portable
-// size), else 8 (queried once, with the most shared memory).
+// CTAs of a cluster: 16 where the device places that many (a non-portable size),
+// else 8, else none (asked once, with the most shared memory).
 int small_cluster() {
   static const int cluster = [] {
-    cudaLaunchAttribute attr;
-    const cudaLaunchConfig_t cfg = small_config(16, kSmallSmem, &attr, 0);
-    int c = 0;
-    if (configure_small() != cudaSuccess || cudaOccupancyMaxActiveClusters(&c, small_kernel(false, true), &cfg) != cudaSuccess) {
+    if (configure_small() != cudaSuccess) {
       cudaGetLastError();
-      c = 0;
+      return 0;
     }
-    return c >= 1 ? 16 : 8;
+    for (const int ctas : {16, 8}) {
+      cudaLaunchAttribute attr;
+      const cudaLaunchConfig_t cfg = small_config(ctas, kSmallSmem, &attr, 0);
+      int c = 0;
+      if (cudaOccupancyMaxActiveClusters(&c, small_kernel(false, true), &cfg) == cudaSuccess && c >= 1) return ctas;
+      cudaGetLastError();
+    }
+    return 0;
   }();
   return cluster;
 }
@@ -583,7 +587,7 @@ int small_cluster() {
 
 bool small_fits(int size, int ctas) {
   const int n = size - 1, cl = ctas ? ctas : small_cluster();
-  if (n < 5 || size > kSmallMaxSize || cl > small_cluster()) return false;
+  if (n < 5 || size > kSmallMaxSize || cl == 0 || cl > small_cluster()) return false;
   return SmallLayout::slots(size, cl - 1) <= kSmallSlots && small_smem(size, cl, false) <= kSmallSmem;
 }
 
