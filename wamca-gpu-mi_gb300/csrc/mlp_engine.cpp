@@ -696,13 +696,19 @@ int JobSet::init() {
   return ensure_list();
 }
 
-// The lists that the set's sweeps can launch from are built with the set and
-// where its shape changes, so that no launch has to, whatever mask, sweep kernel
-// or candidate mode it comes with (under stream capture it could not).  Only a
-// set whose active jobs changed builds the others when they are needed.
+// The list that the set's sweeps launch from is built where mask, shape, sweep
+// kernel and candidate mode are set, so that no launch has to (under stream
+// capture it could not).  A sweep kernel set during a capture finds the other
+// list: launch_dvnd_sweep takes it.
 int JobSet::ensure_list() {
-  const int st = ensure_tiles(0);
-  return st != kOk || !may_sweep64() ? st : ensure_tiles(wide_list());
+  const int list = sweep_list();
+  if (lists_[list].ok) return kOk;
+  if (lists_[1 - list].ok) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    MLP_CUDA(cudaStreamIsCapturing(stream_, &cs), "sweep tiles");
+    if (cs != cudaStreamCaptureStatusNone) return kOk;
+  }
+  return ensure_tiles(list);
 }
 
 int JobSet::ensure_tiles(int list, int buf, bool sync) {
@@ -764,7 +770,7 @@ int JobSet::set_active(const std::vector<int>& idx, int buf, bool sync) {
   MLP_CUDA(cudaMemcpyAsync(djobs_, h, sizeof(JobDev) * jobs_.size(), cudaMemcpyHostToDevice, stream_),
            "copy jobs");
   drop_tiles();
-  return ensure_tiles(dvnd_list(), buf, sync);
+  return ensure_tiles(sweep_list(), buf, sync);
 }
 
 int JobSet::ensure_all_active() {
@@ -932,7 +938,7 @@ int JobSet::set_sweep_kernel(int variant) {
   if (variant == sweep_variant_) return kOk;
   sweep_variant_ = variant;
   drop_graphs();
-  return kOk;
+  return djobs_ ? ensure_list() : kOk;
 }
 
 int JobSet::set_merge_mode(int mode) {
@@ -964,18 +970,22 @@ int JobSet::sweep_only() {
 }
 
 int JobSet::sweep_kernel() {
-  const int st = ensure_tiles(sweep64() ? wide_list() : 0);
+  const int st = ensure_list();
   return st != kOk ? st : launch_dvnd_sweep();
 }
 
 int JobSet::launch_dvnd_sweep() {
-  const TileList& l = lists_[sweep64() ? wide_list() : 0];
-  if (sweep64())
+  // The other list stands in for one that a capture kept from being built: the
+  // general kernel sweeps it to the same keys.
+  const bool own = lists_[sweep_list()].ok;
+  const int list = own ? sweep_list() : 1 - sweep_list();
+  const TileList& l = lists_[list];
+  if (own && sweep64())
     MLP_CUDA(launch_sweep_dvnd_wide(l.d, l.n, djobs_, wide_shape(shape_), stream_), "sweep kernel");
-  else if (dvnd_sweep())
+  else if (own && dvnd_sweep())
     MLP_CUDA(launch_sweep_dvnd(l.d, l.n, djobs_, shape_, local_terms(), stream_), "sweep kernel");
   else
-    MLP_CUDA(launch_sweep(l.d, l.n, djobs_, wide_, shape_, true, stream_), "sweep kernel");
+    MLP_CUDA(launch_sweep(l.d, l.n, djobs_, wide_, list == 1 ? wide_shape(shape_) : shape_, true, stream_), "sweep kernel");
   return kOk;
 }
 
@@ -1006,7 +1016,7 @@ int JobSet::graph_for(int iters, cudaGraphExec_t* out) {
 
 int JobSet::enqueue_iterations(int iters) {
   {
-    const int st = ensure_tiles(dvnd_list());
+    const int st = ensure_tiles(sweep_list());
     if (st != kOk) return st;
   }
   if (stream_ == 0) {
@@ -1076,7 +1086,7 @@ int JobSet::enqueue_device_loop(int max_iters) {
   }
   const int unroll = kDeviceLoopBody;
   {
-    const int st = ensure_tiles(dvnd_list());
+    const int st = ensure_tiles(sweep_list());
     if (st != kOk) return st;
   }
   if (max_iters <= kDirectIters) {
@@ -1156,7 +1166,7 @@ int JobSet::run(int max_iters, bool sync) {
     return read_stats(&s);
   }
   {
-    const int st = ensure_tiles(dvnd_list());
+    const int st = ensure_tiles(sweep_list());
     if (st != kOk) return st;
   }
   MLP_CUDA(launch_stats_begin(djobs_, (int)jobs_.size(), max_iters, stream_), "stats kernel");

@@ -206,7 +206,8 @@ class JobSet {
 
  private:
   // The tile list of a sweep: list 0 in the set's shape, list 1 in the shape
-  // of the 64-bit DVND sweep where that is another one.
+  // of the 64-bit DVND sweep where that is another one.  Built when first
+  // needed; set_active and set_shape invalidate them.
   struct TileList {
     SweepTile* d = nullptr;
     SweepTile* h[2] = {nullptr, nullptr};  // pinned staging
@@ -216,8 +217,8 @@ class JobSet {
   };
   int ensure_list();
   int ensure_tiles(int list, int buf = 0, bool sync = true);
-  int wide_list() const { return wide_shape(shape_) == shape_ ? 0 : 1; }  // the list of the 64-bit DVND sweep
-  int dvnd_list() const { return sweep64() && !total_ ? wide_list() : 0; }  // the list of an iteration's sweep
+  // The list of the selected sweep (TOTAL mode's shapes are the 64-bit sweep's own: list 0).
+  int sweep_list() const { return sweep64() && wide_shape(shape_) != shape_ ? 1 : 0; }
   void drop_tiles() { lists_[0].ok = lists_[1].ok = false; }
   int refuse_capture(const char* what);
   int check_stats(const int64_t* hst);  // the statistics' internal error words

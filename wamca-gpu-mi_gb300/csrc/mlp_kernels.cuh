@@ -131,6 +131,8 @@ cudaError_t launch_sweep_dvnd(const SweepTile* tiles, int ntiles, const JobDev* 
 constexpr int wide_shape(int shape) {
   return kTileShapes[shape].tr >= 16 ? 7 : kTileShapes[shape].tl == 128 ? 6 : kTileShapes[shape].tr == 8 ? 4 : 3;
 }
+static_assert(wide_shape(kTotalShapeSmall) == kTotalShapeSmall && wide_shape(kTotalShapeLarge) == kTotalShapeLarge,
+              "one list serves TOTAL mode's sweeps");
 cudaError_t launch_sweep_dvnd_wide(const SweepTile* tiles, int ntiles, const JobDev* jobs, int shape, cudaStream_t s);
 cudaError_t launch_sweep_collect(const SweepTile* tiles, int ntiles, const JobDev* jobs, bool wide, int shape,
                                  cudaStream_t s);
