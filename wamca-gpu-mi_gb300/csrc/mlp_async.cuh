@@ -20,9 +20,6 @@ __device__ __forceinline__ void mbar_arrive_expect(uint64_t* bar, uint32_t bytes
 // Orders this thread's ordinary shared-memory accesses before later bulk
 // copies to the same bytes.
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
 
 // Copies `bytes` (a multiple of 16) from global to shared memory, both 16-byte
 // aligned; completion is counted on `bar`.

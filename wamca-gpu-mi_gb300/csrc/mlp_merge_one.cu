@@ -13,7 +13,7 @@
 // k_merge_solo runs the five neighbourhoods one after the other.
 //
 // Measured on GB300, cluster merge -> this one, us an iteration of one search:
-// n = 417 16.6 -> 13.0, 700 18.9 -> 15.9, 1000 22.1 -> 19.2, 1999 35.0 -> 34.1;
+// n = 417 16.6 -> 13.0, 700 18.9 -> 15.9, 1000 22.1 -> 19.2, 1999 34.5 -> 34.2;
 // k_merge_solo -> this one, 24 searches of n in [100, 1000] 12.1 -> 9.9 ms, 96
 // 20.7 -> 16.9, 1024 107.5 -> 102.3.  Bound by latency: of n = 1000's 29,600
 // warp instructions most wait for their own fetch (a launch runs its code once;
@@ -86,13 +86,14 @@ template <int PER>
 __device__ __forceinline__ void interval_greedy(int nb, int c, int gtid, int nw, int bar, uint64_t* gmin,
                                                 const uint64_t* lkey, const uint32_t* lab, const MoveList& out) {
   const int lane = gtid & 31, gw = gtid >> 5, stride = 32 * nw;
-  // (delta, block) as two words: the delta's low 32 bits decide 32-bit searches
-  // by themselves; the order is that of the 59-bit key in any case.
+  // (delta, block) as the two words of the key moved to the top of 64 bits:
+  // an improving candidate's key has 45 + 14 bits (the 46th is set for deltas
+  // from zero on, which are no candidates here).
   uint32_t hi[PER], lo[PER], ab[PER];
 #pragma unroll
   for (int q = 0; q < PER; q++) {
     const int x = q * stride + gtid;
-    const uint64_t k = x < c ? lkey[x] << 5 : kKeyNone;  // 46 + 14 bits: the top of 64
+    const uint64_t k = x < c ? lkey[x] << 5 : kKeyNone;
     hi[q] = (uint32_t)(k >> 32);
     lo[q] = (uint32_t)k;
     ab[q] = x < c ? lab[x] & 0xffff7fffu : 0u;

@@ -17,7 +17,7 @@
 // as the two-kernel iteration.
 //
 // Distances: the whole matrix in every sweeping CTA's shared memory where it
-// fits (RESIDENT, up to n = 222), else the CTA's rows, copied anew each
+// fits (RESIDENT, up to n = 223), else the CTA's rows, copied anew each
 // iteration by one bulk copy a row behind the prefix sums.
 //
 // Measured on GB300 (us an iteration of a search from a random start, its host

@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(TL, CAP ? 1024 / TL : 1) k_sweep_dvnd(const Sw
 // rows where some lane improves, the gather's columns are held in registers (no
 // index division, no client reads from shared memory), rows that have no pair
 // left are neither gathered nor evaluated.  1,024 searches of 100..1000 nodes
-// 107.4 -> 95.3 ms, 24 of them 11.0 -> 9.6 (both with their merges).
+// 102.3 -> 95.3 ms, 24 of them 10.8 -> 9.8 (both with their merges).
 template <int TLD, int TR>
 __global__ void __launch_bounds__(TLD / 2) k_sweep_dvnd2(const SweepTile* __restrict__ tiles,
                                                          const JobDev* __restrict__ jobs) {
