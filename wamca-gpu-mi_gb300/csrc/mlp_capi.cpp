@@ -608,6 +608,7 @@ MLP_API int mlp_solver_begin(mlp_solver_t s, int32_t nb_mask, int32_t max_iters)
   if (!s) return arg_error("null solver");
   if (max_iters <= 0) return arg_error("max_iters must be positive");
   MLP_TRY(s->set->set_mask(nb_mask));
+  s->set->limit_run(max_iters);
   MLP_CUDA(launch_stats_begin(s->set->device_jobs(), 1, max_iters, s->set->stream()), "stats kernel");
   return kOk;
 }

@@ -183,6 +183,8 @@ class JobSet {
   JobDev* device_jobs() const { return djobs_; }
   // One DVND iteration over the current jobs (no statistics reset).
   int launch_iteration();
+  // The iterations up to the next call are those of a run of at most max_iters.
+  void limit_run(int max_iters);
   // Merge kernel: kMergeAuto (k_merge_one where merge_one_serves(); else
   // k_merge_solo for sets of kSoloMinJobs jobs or more, a six-CTA cluster per
   // job otherwise), kMergeCluster, kMergeSolo.
@@ -234,6 +236,8 @@ class JobSet {
   // critical path) write term tables.
   bool local_terms() const { return all_jobs_.size() == 1; }
   bool small_search() const;
+  static constexpr int kEarlySize = 600;
+  bool cluster_early() const;
   int launch_dvnd_sweep();
   int graph_for(int iters, cudaGraphExec_t* out);
   std::vector<Job*> all_jobs_;  // every job of the set (statistics order)
@@ -263,8 +267,10 @@ class JobSet {
   int64_t* dstats_ = nullptr;  // device, kStatWords per job (jobs' stats live here)
   std::vector<void*> extra_ws_;  // merge workspaces allocated for jobs of mixed-size sets
   std::map<int, cudaGraphExec_t> graphs_;
-  cudaGraphExec_t loop_graph_ = nullptr;
-  int loop_unroll_ = 0;
+  cudaGraphExec_t loop_graph_[2] = {nullptr, nullptr};  // by early_
+  // The run is limited to its searches' first iterations (a twelfth of their
+  // positions), in which most blocks have an improving candidate.
+  bool early_ = false;
 };
 
 // Start tours of MLSolution::random built on the device (mlp_grasp.cu), one
