@@ -149,8 +149,9 @@ MLP_API int mlp_solver_set_sweep_kernel(mlp_solver_t s, int32_t variant);
  * (-1, the default: 2^20 times, a second or more).  Results are identical. */
 MLP_API int mlp_solver_set_small_search(mlp_solver_t s, int32_t ctas, int32_t polls);
 /* Merge kernel of the solver's iterations (as mlp_batch_set_merge_mode; the
- * default for one search is one CTA up to 1,999 nodes, then the six-CTA
- * cluster).  Every mode gives the same results. */
+ * default for one search is one CTA up to 1,999 nodes, and the six-CTA cluster
+ * above them and in runs limited to a search's first iterations).  Every mode
+ * gives the same results. */
 MLP_API int mlp_solver_set_merge_mode(mlp_solver_t s, int32_t mode);
 /* Candidate mode of every later pass / DVND of this solver.  0 (default): one
  * candidate per reference block (the ODC kernels).  1: TOTAL multi-improvement
