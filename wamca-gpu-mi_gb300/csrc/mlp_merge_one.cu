@@ -32,6 +32,12 @@ namespace {
 // Largest tour (positions; see merge_one_serves): a neighbourhood has fewer
 // candidates.
 constexpr int kOneMaxSize = 2000;
+// Positions that the threads' arrays hold, which is a matter of the code the
+// compiler makes of them: us an iteration at n = 420, 700, 850, 1000 with 2,008 |
+// 2,120, in 32 bits 13.12 16.32 17.28 19.57 | 13.02 16.17 17.15 19.47, in 64
+// bits 13.35 16.48 17.49 19.89 | 13.52 16.68 17.67 20.08.
+template <bool WIDE>
+constexpr int kOneItems = WIDE ? kOneMaxSize + 8 : 2120;
 
 // Shared memory (bytes): the stage-3 list, then the candidate lists and swap
 // tables of stage 2, under which the conflict rows, the position map, the old
@@ -218,7 +224,7 @@ __device__ __forceinline__ void swap_tables(int sz, int c, int gtid, int gnt, in
 template <bool WIDE, int NT>
 __device__ __forceinline__ void one_rebuild(const JobDev* J, int sz, const int32_t* t, int32_t* w_s, const int32_t* src) {
   using C = typename Arith<WIDE>::C;
-  constexpr int PER = (kOneMaxSize + 8 + NT - 1) / NT, nw = NT / 32;
+  constexpr int PER = (kOneItems<WIDE> + NT - 1) / NT, nw = NT / 32;
   __shared__ C s_w[PER * nw], s_q[PER * nw];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, n = J->n, pad = sz + 8;
   const int32_t* __restrict__ D = J->D;
@@ -372,7 +378,7 @@ __global__ void __launch_bounds__(NT) k_merge_one(const JobDev* __restrict__ job
   if (tid < (int)(sizeof(JobDev) / 8)) ((uint64_t*)&s_job)[tid] = ((const uint64_t*)Jg)[tid];
   // The current tour, in registers until stage 2 is over.
   const int32_t* tour = Jg->tour;
-  constexpr int kTourPer = (kOneMaxSize + 8 + NT - 1) / NT;
+  constexpr int kTourPer = (kOneItems<WIDE> + NT - 1) / NT;
   int32_t mine[kTourPer];
 #pragma unroll
   for (int u = 0; u < kTourPer; u++) mine[u] = tid + u * nt < sz ? tour[tid + u * nt] : 0;
@@ -547,12 +553,11 @@ cudaError_t configure_merge_one() {
 
 // Where this merge serves, all limits in positions.  One search: up to 2,000
 // (merge_one_max_size(); 2,115 would fit its shared memory).  Us an iteration,
-// this merge | the cluster's: n = 1100 22.6 | 24.5, 1500 27.0 | 28.3, 1700 29.2 |
-// 29.8, 1900 33.3 | 33.3, 1999 34.2 | 34.5; 64-bit 1100 23.5 | 25.1, 1500 36.5 |
-// 39.9, 1700 40.8 | 41.1, 1999 42.8 | 43.1.  The longer the lists, the less the
-// cluster's hand-off counts: built for 2,115, with a third position a thread, it
-// took 36.0 | 35.9 at 2050 and 37.5 | 37.1 at 2114, 64-bit 44.8 | 44.2 and 45.8 |
-// 45.0.
+// this merge | the cluster's: n = 1100 22.8 | 24.5, 1500 27.2 | 28.3, 1700 29.4 |
+// 29.8, 1999 34.3 | 34.4; 64-bit 1100 23.5 | 25.1, 1500 36.5 | 39.9, 1700 40.8 |
+// 41.1, 1999 42.8 | 43.1.  The longer the lists, the less the cluster's hand-off
+// counts: it took 36.0 | 35.9 at 2050 and 37.5 | 37.1 at 2114, 64-bit 44.8 | 44.2
+// and 45.8 | 45.0.
 // Several searches: while the layout takes at most 113 KB (1,094 positions).  Its
 // CTAs run one an SM at any size (1,024 threads of 64 registers); of larger
 // layouts the sweep seems to suffer, whose CTAs and L1 cache share what a merge
